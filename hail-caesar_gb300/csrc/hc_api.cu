@@ -730,6 +730,7 @@ static hc_status device_error(hc_ctx* c) {
   const int e = c->hdev->err_code;
   if (e == 301) return hc_fail(c, HC_ERR_NONFINITE, "non-finite water depth (device error 301)");
   if (e == 401) return hc_fail(c, HC_ERR_TIMEOUT, "drainage sweep: a device wait gave up (401)");
+  if (e == 402) return hc_fail(c, HC_ERR_TIMEOUT, "creep: a device wait gave up (402)");
   return hc_fail(c, HC_ERR_STATE, "device error %d", e);
 }
 

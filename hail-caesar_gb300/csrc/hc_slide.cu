@@ -3,7 +3,8 @@
 //   global_landsliding     :5529-5654 (daily: the same probe and warp replay
 //                          over every cell, sweep after sweep, or a skewed
 //                          wavefront when most cells move)
-//   creep                  :5293-5427 (host-driven, every 10 days)
+//   creep                  :5293-5427 (host-driven, every 10 days; its grain
+//                          transfers as a wavefront of rows)
 //
 // slide_3 is a sequential relaxation: every test sees the elevations left by
 // the moves before it, in the reference's loop order.  Moves are rare (a
@@ -193,15 +194,15 @@ __global__ void k_slide_probe(const hc_view c, const hc_dev* d, uint8_t* flag, d
   flag[o.pos(x, y)] = f;
 }
 
-// Per-block counts of the flags; the block that finishes last scans them
-// (exclusive, in place) and stores the total.
+// Per-block counts of the flags (set bits of each byte); the block that
+// finishes last scans them (exclusive, in place) and stores the total.
 __global__ void __launch_bounds__(1024) k_flag_count(const uint8_t* flag, size_t n,
                                                      int32_t* block_sums, int32_t* total,
                                                      hc_dev* d, int gated) {
   __shared__ int ws[32];
   if (gated && !(d->it_active && d->rest_active && d->do_slide)) return;
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  int v = (i < n) ? flag[i] : 0;
+  int v = (i < n) ? __popc(flag[i]) : 0;
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = v;
   __syncthreads();
@@ -711,20 +712,266 @@ __global__ void k_creep_gather(const hc_view c, double* tempcreep, double time) 
   tempcreep[(size_t)x * c.W + y] = t;
 }
 
-// grain transfers of creep, serial (only cells holding a grain record move
-// grain, and a receiver may get its first record)
-__global__ void k_creep_grain(const hc_view c, hc_dev* d, double time) {
-  const int cx[8] = {0, 1, 1, 1, 0, -1, -1, -1};
-  const int cy[8] = {-1, -1, 0, 1, 1, 1, 0, -1};
-  for (int x = 2; x <= c.imax - 1; x++)
-    for (int y = 2; y <= c.jmax - 1; y++) {
-      const size_t cell = (size_t)x * c.W + y;
-      if (c.index[cell] == -9999) continue;
-      for (int k = 0; k < 8; k++) {
-        double v = creep_temp(c, x, y, k, time);
-        if (v >= 0) slide_GS_dev(c, d, cell, v, (size_t)(x + cx[k]) * c.W + (y + cy[k]), true);
+// Grain transfers of creep.  The reference's loop visits the cells row by
+// row; a cell that holds a record slides grain to its lower neighbours in
+// turn, and a receiver without a record gets one.  A visit reads and changes
+// records of its 3x3 block only (elevations and bedrock are those before the
+// creep throughout), so two visits conflict only when their rows and their
+// columns each differ by at most 2.  One warp takes a row and walks it in
+// order, never nearer than three columns behind the row above: then every
+// visit comes after all earlier ones that it conflicts with, and the records
+// are the serial loop's.  Rows are handed out in order by a counter, so the
+// topmost unfinished row is always held by a running warp and never waits
+// for one that is not; every wait is bounded all the same.
+//
+// Within a visit lane n holds fraction n of the records (the serial sums over
+// the fractions keep their order: every lane forms the same sum), and the
+// moves of four cells are formed ahead, one per lane.
+//
+// What bounds it is the chain of visits: about jmax + 3 imax of them, one
+// slide after another, each a sum of nine dependent additions, a quotient and
+// two record checks.  One thread for the whole grid took 22 us a cell (890 ms
+// at 200 x 200, 5.9 s at 512 x 512); the rows take about 9 ms at 200 x 200.
+//
+// New records are numbered afterwards: a visit marks the directions that made
+// one (in its own byte of `made`), and their order in the serial loop is the
+// order of (cell, direction).
+constexpr int kCreepWarps = 4;           // rows per block
+constexpr long kCreepSpins = 1L << 22;   // polls before a wait gives up (seconds)
+
+struct CreepSync {
+  unsigned int ticket;  // rows handed out
+  unsigned int err;     // a wait ran out
+  unsigned int pad[14];
+  int done[1];          // per row: last column visited
+};
+
+// sort_active :3874-3947 on the record held by the warp (plane L in lane L);
+// values other warps may have written are read past L1
+static __device__ void creep_sort(const hc_view& c, size_t cell, double& g) {
+  const int L = threadIdx.x & 31;
+  const double active = c.p.active;
+  const float f = (L <= HC_G) ? approx_f(g) : 0.0f;
+  float sf = f, af = fabsf(f);
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) {  // lanes 0..15 hold all of them
+    sf += __shfl_xor_sync(kFull, sf, o);
+    af += __shfl_xor_sync(kFull, af, o);
+  }
+  sf = __shfl_sync(kFull, sf, 0);
+  af = __shfl_sync(kFull, af, 0);
+  const float tol = 1e-5f * af + 1e-30f;
+  const float hi = c.act_hi, lo = c.act_lo;
+  const int dep = (sf > hi + tol) ? 1 : ((sf < hi - tol) ? -1 : 0);
+  const int ero = (sf < lo - tol) ? 1 : ((sf > lo + tol) ? -1 : 0);
+  if (dep == -1 && ero == -1) return;
+  double total = 0.0;  // in the reference's order, n = 0 .. HC_G
+  for (int n = 0; n <= HC_G; n++) total += __shfl_sync(kFull, g, n);
+  if (total > (active * 1.5)) {
+    if (L <= HC_G - 2) {
+      double z0[9];
+#pragma unroll
+      for (int z = 0; z < 9; z++) z0[z] = __ldcg(&STR(c, cell, z, L));
+#pragma unroll
+      for (int z = 0; z < 9; z++) __stcg(&STR(c, cell, z + 1, L), z0[z]);
+    }
+    __syncwarp();
+    const double coeff = active / total;
+    if (L >= 1 && L <= HC_G - 1 && g > 0.0) {
+      const double amount = coeff * g;
+      __stcg(&STR(c, cell, 0, L - 1), amount);
+      g = g - amount;
+    }
+    __syncwarp();
+  }
+  if (total < (active / 4)) {
+    double s0 = 0;
+    if (L >= 1 && L <= HC_G - 1) s0 = __ldcg(&STR(c, cell, 0, L - 1));
+    __syncwarp();
+    if (L <= HC_G - 2) {
+      double z0[9];
+#pragma unroll
+      for (int z = 0; z < 9; z++) z0[z] = __ldcg(&STR(c, cell, z + 1, L));
+#pragma unroll
+      for (int z = 0; z < 9; z++) __stcg(&STR(c, cell, z, L), z0[z]);
+    }
+    __syncwarp();
+    if (L >= 1 && L <= HC_G - 1) {
+      g += s0;
+      __stcg(&STR(c, cell, 9, L - 1), active * c.p.dprop[L]);
+    }
+    __syncwarp();
+  }
+}
+
+// slide_GS :4077-4171 from a cell's record (a) to a neighbour's (b), both
+// held by the warp; made: b has no record yet and gets one
+static __device__ void creep_slide(const hc_view& c, size_t acell, double& a, double amount,
+                                   size_t bcell, double& b, bool make) {
+  const int L = threadIdx.x & 31;
+  const bool fr = L >= 1 && L <= HC_G - 1;
+  const double dp = fr ? c.p.dprop[L] : 0.0, active = c.p.active;
+  if (make) {  // addGS :3949-3983
+    b = fr ? active * dp : 0.0;
+    if (L <= HC_G - 2) {
+      const double elev = c.elev[bcell], bed = c.bed[bcell], s = active * c.p.dprop[L + 1];
+      for (int z = 0; z <= 9; z++) {
+        const bool below = elev - (active * (z + 1)) < (bed - active);
+        __stcg(&STR(c, bcell, z, L), below ? 0.0 : s);
       }
     }
+    __syncwarp();
+    if (amount > active) {
+      if (fr) b += amount * dp;
+      amount = active;
+    }
+  }
+  double total = 0;  // positive fractions 1..9, in order
+#pragma unroll
+  for (int n = 1; n <= HC_G - 1; n++) {
+    const double v = __shfl_sync(kFull, a, n);
+    if (dgt0(v)) total += v;
+  }
+  if (!make && amount > total) {
+    if (fr) b += (amount - total) * dp;
+    amount = total;
+  }
+  if (dgt0(total) && fr) {
+    const double t = amount * ddiv_rn(a, total);
+    b += t;
+    double na = a;
+    if (!make || na > 0.0001) na -= t;
+    if (dlt0(na)) na = 0;
+    a = na;
+  }
+  creep_sort(c, acell, a);
+  creep_sort(c, bcell, b);
+}
+
+__global__ void __launch_bounds__(32 * kCreepWarps) k_creep_grain(const hc_view c, hc_dev* d,
+                                                                  CreepSync* sync, uint8_t* made,
+                                                                  double time) {
+  const int cx[8] = {0, 1, 1, 1, 0, -1, -1, -1};
+  const int cy[8] = {-1, -1, 0, 1, 1, 1, 0, -1};
+  const int L = threadIdx.x & 31;
+  const size_t W = c.W;
+  const int last = c.jmax - 1;
+  for (;;) {
+    unsigned ticket = 0;
+    if (L == 0) ticket = atomicAdd(&sync->ticket, 1u);
+    ticket = __shfl_sync(kFull, ticket, 0);
+    if (ticket >= (unsigned)(c.imax - 2)) return;
+    const int x = 2 + (int)ticket;
+    const volatile int* above = &sync->done[x - 1];
+    volatile int* mine = &sync->done[x];
+    int seen = (x == 2) ? INT_MAX : 0;  // last column the row above is known to have visited
+    double v = -1;
+    unsigned moves = 0;
+    for (int y = 2; y <= last; y++) {
+      const int q = (y - 2) & 3;
+      if (q == 0) {  // the moves of cells y .. y+3
+        const int yy = y + (L >> 3);
+        v = yy <= last ? creep_temp(c, x, yy, L & 7, time) : -1.0;
+        moves = __ballot_sync(kFull, v >= 0);
+      }
+      const int need = min(y + 2, last);
+      if (seen < need) {
+        int got = 0;
+        if (L == 0) {
+          long spins = 0;
+          while ((got = *above) < need) {
+            if (++spins > kCreepSpins || *(volatile unsigned*)&sync->err) {
+              atomicExch(&sync->err, 1u);
+              got = -1;
+              break;
+            }
+          }
+          __threadfence();
+        }
+        seen = __shfl_sync(kFull, got, 0);
+        if (seen < 0) {  // gave up: the records are not complete
+          if (L == 0) {
+            d->err_code = 402;
+            atomicOr((unsigned int*)&d->pause, HC_PAUSE_ERROR);
+          }
+          return;
+        }
+      }
+      const unsigned m = (moves >> (8 * q)) & 0xffu;
+      const size_t cell = (size_t)x * W + y;
+      if (m && __ldcg(&c.index[cell]) != -9999) {
+        // the cell's and its receivers' records, loaded together
+        const size_t mynb = (size_t)(x + cx[L & 7]) * W + (y + cy[L & 7]);
+        const int nidx = (L < 8) ? __ldcg(&c.index[mynb]) : 0;
+        double a = (L <= HC_G) ? __ldcg(&GRN(c, cell, L)) : 0.0;
+        double b[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+          const size_t nb = (size_t)(x + cx[k]) * W + (y + cy[k]);
+          b[k] = (((m >> k) & 1u) && L <= HC_G) ? __ldcg(&GRN(c, nb, L)) : 0.0;
+        }
+        const unsigned none = __ballot_sync(kFull, L < 8 && nidx == -9999) & m;
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+          if (!((m >> k) & 1u)) continue;
+          const size_t nb = (size_t)(x + cx[k]) * W + (y + cy[k]);
+          creep_slide(c, cell, a, __shfl_sync(kFull, v, 8 * q + k), nb, b[k], (none >> k) & 1u);
+        }
+        if (L <= HC_G) {
+          __stcg(&GRN(c, cell, L), a);
+#pragma unroll
+          for (int k = 0; k < 8; k++)
+            if ((m >> k) & 1u)
+              __stcg(&GRN(c, (size_t)(x + cx[k]) * W + (y + cy[k]), L), b[k]);
+        }
+        if (L < 8 && ((none >> L) & 1u)) __stcg(&c.index[mynb], -2);  // number pending
+        if (L == 0 && none) made[cell] = (uint8_t)none;
+        __syncwarp();
+        if (L == 0) __threadfence();
+      }
+      if (L == 0) *mine = y;
+    }
+  }
+}
+
+// Numbers the records the visits made: block_sums as k_flag_count left them,
+// the bytes' set bits counted in cell order.
+__global__ void __launch_bounds__(1024) k_creep_number(const hc_view c, const hc_dev* d,
+                                                       const uint8_t* made,
+                                                       const int32_t* block_sums) {
+  const int cx[8] = {0, 1, 1, 1, 0, -1, -1, -1};
+  const int cy[8] = {-1, -1, 0, 1, 1, 1, 0, -1};
+  __shared__ int ws[32];
+  __shared__ int wb[32];
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  unsigned m = (i < c.N2) ? made[i] : 0u;
+  const int v = __popc(m);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int incl = v;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int t = __shfl_up_sync(kFull, incl, o);
+    if (lane >= o) incl += t;
+  }
+  if (lane == 31) ws[warp] = incl;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int s = 0;
+    for (int k = 0; k < 32; k++) {
+      wb[k] = s;
+      s += ws[k];
+    }
+  }
+  __syncthreads();
+  int number = d->grain_tot + 1 + block_sums[blockIdx.x] + wb[warp] + incl - v;
+  while (m) {
+    const int k = __ffs(m) - 1;
+    m &= m - 1;
+    c.index[(size_t)((long long)i + cx[k] * (long long)c.W + cy[k])] = number++;
+  }
+}
+
+__global__ void k_creep_total(hc_dev* d, const int32_t* count) {
+  d->grain_tot += *count;
   d->s.grain_array_tot = d->grain_tot;
 }
 
@@ -853,7 +1100,21 @@ hc_status run_creep(hc_ctx* c, double time) {
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->s);
   if (e != cudaSuccess) return hc_cuda(c, e, "creep");
   // grain transfers read the elevations before the creep is applied
-  if (h_any) k_creep_grain<<<1, 1, 0, c->s>>>(c->v, c->dev, time);
+  if (h_any) {
+    SlideScratch sc = slide_scratch(c);
+    const size_t n = c->v.N2;
+    const int nblocks = (int)((n + 1023) / 1024), rows = c->v.imax - 2;
+    // the rows' progress lives in the drainage frontier, which is idle here
+    CreepSync* sync = (CreepSync*)c->v.drain_f0;
+    cudaMemsetAsync(sync, 0, sizeof(CreepSync) + (size_t)(c->v.imax + 2) * sizeof(int), c->s);
+    cudaMemsetAsync(sc.flag, 0, n, c->s);
+    k_creep_grain<<<(rows + kCreepWarps - 1) / kCreepWarps, 32 * kCreepWarps, 0, c->s>>>(
+        c->v, c->dev, sync, sc.flag, time);
+    k_flag_count<<<nblocks, 1024, 0, c->s>>>(sc.flag, n, sc.block_sums, sc.count, c->dev, 0);
+    k_creep_number<<<nblocks, 1024, 0, c->s>>>(c->v, c->dev, sc.flag, sc.block_sums);
+    k_creep_total<<<1, 1, 0, c->s>>>(c->dev, sc.count);
+    count_launch(c, 4);
+  }
   k_creep_apply<<<g, b, 0, c->s>>>(c->v, tempcreep);
   count_launch(c, 1);
   return HC_OK;
