@@ -9,12 +9,12 @@
 // plus the pushes of its higher neighbours, added in the order those were
 // swept.  Here the same sums are pulled instead: a cell is ready once all
 // its higher neighbours are done (Kahn's algorithm on the "higher than"
-// graph), one frontier of ready cells per step, and each cell adds its
-// neighbours' terms in their sweep order (the position in the sort, so equal
-// elevations keep the reference's order).  Every term and every addition is
-// the reference's, so the areas are bit-identical.  Cells the reference's
-// loop never reaches (sorted position 0 and above imax*jmax, where the sort's
-// padding pairs push them) keep area 0 and push nothing, as there.
+// graph), and it adds its neighbours' terms in their sweep order (the
+// position in the sort, so equal elevations keep the reference's order).
+// Every term and every addition is the reference's, so the areas are
+// bit-identical.  Cells the reference's loop never reaches (sorted position 0
+// and above imax*jmax, where the sort's padding pairs push them) keep area 0
+// and push nothing, as there.
 //
 // The sort itself is needed only where its order among equal elevations can
 // show: two higher neighbours of one cell at the same elevation (the order
@@ -140,7 +140,7 @@ __global__ void k_drain_pos(const hc_view c, const uint32_t* __restrict__ order)
   }
 }
 
-// per interior cell: area = 0, the sum of downhill drops (difftot, the
+// per interior cell: the sum of downhill drops (difftot, the
 // reference's clamped 8-neighbour loop in its order), the number of higher
 // neighbours to wait for (cells with none start the first frontier), whether
 // the sweep reaches the cell (drain_pos 1/0: below the selected last
@@ -152,7 +152,6 @@ __global__ void k_drain_init(const hc_view c, hc_dev* d, const double* __restric
   const size_t W = c.W;
   const size_t cell = (size_t)i * W + j;
   const double e = el[cell];
-  c.area[cell] = 0;
   double difftot = 0;
   for (int dir = 1; dir <= 8; dir++) {
     const int i2 = clampi(i + kDrX[dir], 1, c.imax), j2 = clampi(j + kDrY[dir], 1, c.jmax);
@@ -184,326 +183,358 @@ __global__ void k_drain_init(const hc_view c, hc_dev* d, const double* __restric
   const bool reached = !(u > a->prefix) &&
                        !(a->min_u < kZeroKey && a->min_count == 1 && u == a->min_u);
   c.drain_pos[cell] = reached ? 1u : 0u;
-  if (higher == 0) {
-    const unsigned k = atomicAdd(&d->drain_front, 1u);
-    c.drain_f0[k] = (uint32_t)cell;
+  // one atomic per warp
+  const unsigned act = __activemask(), m = __ballot_sync(act, higher == 0);
+  if (m) {
+    const unsigned lane = threadIdx.x & 31;
+    const int leader = __ffs(act) - 1;
+    unsigned base = 0;
+    if ((int)lane == leader) base = atomicAdd(&d->drain_front, (unsigned)__popc(m));
+    base = __shfl_sync(act, base, leader);
+    if (higher == 0) c.drain_f0[base + __popc(m & ((1u << lane) - 1u))] = (uint32_t)cell;
   }
 }
 
-// The share of each higher neighbour's area that reaches this cell, before
-// the sweep: the reference's term (e_q - e)/difftot_q, or its diagonal form
-// ((e_q - e)/1.414)/difftot_q, for the first direction of q whose (clamped)
-// step lands here; neighbours with more than one such direction (at the
-// edges) are marked and summed term by term in the sweep.  The sweep then
-// adds aq * share, the reference's operations on the same values, and its
+// A cell's terms, before the sweep: its higher neighbours that the sweep
+// reaches, in sweep order (higher elevation first, equal elevations by sorted
+// position), each with the share of its area that comes here: the
+// reference's term (e_q - e)/difftot_q, or its diagonal form
+// ((e_q - e)/1.414)/difftot_q, per direction of q whose (clamped) step lands
+// here, in the order of the directions (one for an interior q, possibly two
+// at the edges; never more than eight terms in all).  The sweep then adds
+// area_q * share, the reference's operations on the same values, and its
 // critical path has no division (about 600 cycles each on this GPU's FP64
-// pipe, against 128 for a multiply and an add).
-__global__ void k_drain_frac(const hc_view c, const double* __restrict__ el) {
+// pipe, against 128 for a multiply and an add) and no ordering to find.
+//
+// drain_head of a cell: 4 bits per term with the neighbour's number
+// 3*(di+1) + (dj+1), their count at bit 32, the mask of its lower neighbours
+// (by number) at bit 36, bit 45 when the sweep reaches it, bit 46 when its
+// own unit of area counts (not no-data).
+constexpr int kHeadCount = 32, kHeadLower = 36, kHeadReached = 45, kHeadOwn = 46;
+
+__global__ void k_drain_terms(const hc_view c, const double* __restrict__ el) {
   int i, j;
   if (!interior_ij(c, i, j)) return;
-  const size_t W = c.W, N2 = c.N2;
+  const size_t W = c.W;
   const size_t cell = (size_t)i * W + j;
   const double e = el[cell];
-  unsigned multi = 0;
-  for (int kk = 0; kk < 9; kk++) {
-    double g = 0;
-    const int iq = i + kk / 3 - 1, jq = j + kk % 3 - 1;
-    if (kk != 4 && iq >= 1 && iq <= c.imax && jq >= 1 && jq <= c.jmax) {
-      const size_t q = (size_t)iq * W + jq;
-      const double eq = el[q];
-      if (eq > e) {
-        const double dq = c.drain_dt[q];
-        int found = 0;
-        for (int dir = 1; dir <= 8; dir++) {
-          const int i3 = clampi(iq + kDrX[dir], 1, c.imax), j3 = clampi(jq + kDrY[dir], 1, c.jmax);
-          if (i3 != i || j3 != j) continue;
-          if (found == 0) g = (dir % 2 != 0) ? ((eq - e) / dq) : (((eq - e) / 1.414) / dq);
-          found++;
-        }
-        if (found > 1) multi |= 1u << kk;
-      }
-    }
-    c.drain_frac[(size_t)kk * N2 + cell] = g;
-  }
-  c.drain_multi[cell] = (uint16_t)multi;
-}
-
-// Grid-wide barrier for k_drain_sweep, which is launched cooperatively (all
-// blocks resident).  Sense by generation count; every wait is bounded: a
-// block that gives up raises err and the sweep ends with an error status.
-struct DrainSync {
-  unsigned int arrive;
-  unsigned int gen;
-  unsigned int err;
-  unsigned int count[3];  // frontier lengths, rotating by level
-  unsigned int solo_level;            // level at which block 0 left its last solo run
-  unsigned int pad;
-  unsigned long long solo_done;       // cells done by then
-};
-
-// Frontiers of at most this many cells are swept by block 0 alone, level
-// after level with block barriers, while the other blocks wait: most
-// frontiers of a catchment hold a few hundred cells, and a grid barrier per
-// level costs more than the work.
-constexpr unsigned kSoloMax = 2048;
-
-// `limit`: spins before giving up; `expect`: arrivals that open it (the
-// number of blocks, unless a test asks for more)
-__device__ __forceinline__ bool grid_barrier(DrainSync* g, unsigned expect, long limit) {
-  __shared__ bool ok;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    ok = true;
-    const unsigned my = *(volatile unsigned*)&g->gen;
-    __threadfence();
-    if (atomicAdd(&g->arrive, 1u) == expect - 1) {
-      g->arrive = 0;
-      __threadfence();
-      atomicAdd(&g->gen, 1u);
-    } else {
-      long spins = 0;
-      while (*(volatile unsigned*)&g->gen == my) {
-        if (++spins > limit || *(volatile unsigned*)&g->err) {
-          atomicExch(&g->err, 1u);
-          ok = false;
-          break;
-        }
-      }
-    }
-    __threadfence();
-  }
-  __syncthreads();
-  return ok;
-}
-
-// One ready cell: pull the pushes of its higher neighbours in sweep order,
-// then count down its lower neighbours.  Returns the neighbours (bit
-// k = 3*(di+1) + (dj+1)) this released into the next frontier.  Values
-// written by other blocks in earlier frontiers are read past L1.
-__device__ unsigned drain_cell_g(const hc_view& c, const double* __restrict__ el,
-                                 uint32_t cell) {
-  const int W = (int)c.W;
-  const int i = (int)(cell / W), j = (int)(cell % W);
-  const double e = el[cell];
-  // every neighbour's elevation, sweep position, area and share of its
-  // area that comes here, loaded together (one round trip)
-  // (elevations as their integer keys: out-of-grid entries take e's)
-  const long long ke = dkey(e);
-  long long ek[9];
-  double an[9], gn[9];
+  unsigned left = 0, lower = 0;
+  double en[9];
   uint32_t pn[9];
 #pragma unroll
   for (int k = 0; k < 9; k++) {
-    const int i2 = i + k / 3 - 1, j2 = j + k % 3 - 1;
-    const bool in = !(i2 < 1 || i2 > c.imax || j2 < 1 || j2 > c.jmax);
-    const size_t q = (size_t)i2 * W + j2;
-    ek[k] = in ? dkey(__ldg(&el[q])) : ke;
-    pn[k] = in ? __ldg(&c.drain_pos[q]) : 0u;
-    an[k] = in ? __ldcg(&c.area[q]) : 0.0;
-    gn[k] = __ldg(&c.drain_frac[(size_t)k * c.N2 + cell]);
+    const int iq = i + k / 3 - 1, jq = j + k % 3 - 1;
+    const bool in = k != 4 && iq >= 1 && iq <= c.imax && jq >= 1 && jq <= c.jmax;
+    const size_t q = (size_t)iq * W + jq;
+    en[k] = in ? el[q] : e;
+    pn[k] = in ? c.drain_pos[q] : 0u;
+    if (en[k] > e && pn[k] != 0) left |= 1u << k;
+    if (en[k] < e) lower |= 1u << k;
   }
-  const unsigned multi = __ldg(&c.drain_multi[cell]);
-  if (pn[4] != 0) {
-    double a = (e == -9999) ? 0.0 : 1.0;
-    // higher neighbours the sweep reached, taken in sweep order: higher
-    // elevation first, equal elevations by sorted position (only in sorted
-    // runs).  Each is picked by a scan with constant indices, so the
-    // neighbour values stay in registers (indexed arrays went to local
-    // memory, which at this block size lives in L2).
-    unsigned left = 0;
-#pragma unroll
-    for (int kk = 0; kk < 9; kk++)
-      if (kk != 4 && ek[kk] > ke && pn[kk] != 0) left |= 1u << kk;
+  const bool reached = c.drain_pos[cell] != 0;
+  unsigned long long head = ((unsigned long long)lower << kHeadLower) |
+                            ((unsigned long long)reached << kHeadReached) |
+                            ((unsigned long long)(e != -9999) << kHeadOwn);
+  int n = 0;
+  if (reached) {
+    double* share = c.drain_share + cell * 8;
 #pragma unroll 1
     while (left) {
       int best = -1;
-      long long bk = 0;
-      unsigned bp = 0;
-      double aq = 0, gq = 0;
+      double be = 0;
+      uint32_t bp = 0;
 #pragma unroll
-      for (int kk = 0; kk < 9; kk++) {
-        if (!((left >> kk) & 1u)) continue;
-        if (best < 0 || ek[kk] > bk || (ek[kk] == bk && pn[kk] > bp)) {
-          best = kk;
-          bk = ek[kk];
-          bp = pn[kk];
-          aq = an[kk];
-          gq = gn[kk];
+      for (int k = 0; k < 9; k++) {
+        if (!((left >> k) & 1u)) continue;
+        if (best < 0 || en[k] > be || (en[k] == be && pn[k] > bp)) {
+          best = k;
+          be = en[k];
+          bp = pn[k];
         }
       }
       left &= ~(1u << best);
-      if (!((multi >> best) & 1u)) {  // one direction of q lands here
-        a += aq * gq;
-        continue;
-      }
       const int iq = i + best / 3 - 1, jq = j + best % 3 - 1;
-      const double dq = c.drain_dt[(size_t)iq * W + jq], eq = el[(size_t)iq * W + jq];
-      // the directions of q whose (clamped) step lands here, in order: one
-      // for an interior q, possibly more at the edges; found with integer
-      // tests first, so that the divisions run once per term and not once
-      // per direction of the warp's slowest lane
-      unsigned dirs = 0;
+      const double dq = c.drain_dt[(size_t)iq * W + jq];
 #pragma unroll 1
       for (int dir = 1; dir <= 8; dir++) {
         const int i3 = clampi(iq + kDrX[dir], 1, c.imax), j3 = clampi(jq + kDrY[dir], 1, c.jmax);
-        if (i3 == i && j3 == j) dirs |= 1u << dir;
-      }
-      while (dirs) {
-        const int dir = __ffs(dirs) - 1;
-        dirs &= dirs - 1;
-        if (dir % 2 != 0)
-          a += aq * ((eq - e) / dq);
-        else
-          a += aq * (((eq - e) / 1.414) / dq);
+        if (i3 != i || j3 != j) continue;
+        share[n] = (dir % 2 != 0) ? ((be - e) / dq) : (((be - e) / 1.414) / dq);
+        head |= (unsigned long long)best << (4 * n);
+        n++;
       }
     }
-    if (a > 0) __stcg(&c.area[cell], a);
   }
-  // No fence here: the area is read by the lower neighbours in a later
-  // frontier, after a block barrier (block 0 alone) or a grid barrier, which
-  // order it before those reads.
-  // the eight decrements do not depend on one another: issue them together
-  int old[9];
-#pragma unroll
-  for (int kk = 0; kk < 9; kk++) {
-    const int dx = kk / 3 - 1, dy = kk % 3 - 1;
-    old[kk] = (kk != 4 && ek[kk] < ke) ? atomicSub(&c.drain_pend[(i + dx) * W + (j + dy)], 1) : 0;
-  }
-  unsigned released = 0;
-#pragma unroll
-  for (int kk = 0; kk < 9; kk++) released |= (old[kk] == 1 ? 1u : 0u) << kk;
-  return released;
+  c.drain_head[cell] = head | ((unsigned long long)n << kHeadCount);
+  // not yet summed: no area is a NaN
+  c.area[cell] = __longlong_as_double(-1LL);
 }
 
-// Sweeps one frontier, the threads of [start, start + stride) taking cells
-// start, start + stride, ...; released cells go to fout, counted in *n_out
-// (one atomic per warp).
-__device__ __forceinline__ void drain_frontier(const hc_view& c, const double* __restrict__ el,
-                                               const uint32_t* fin, unsigned n_in,
-                                               uint32_t* fout, unsigned* n_out, unsigned start,
-                                               unsigned stride) {
+// The sweep's shared state, all zero at the start but `tail`.
+struct DrainSync {
+  unsigned long long done;  // cells finished
+  unsigned int tail;        // queue entries appended
+  unsigned int taken;       // queue entries handed out
+  unsigned int hops;        // cells on the longest chain of releases
+  unsigned int err;         // a wait ran out
+};
+
+constexpr int kSweepThreads = 128;
+constexpr int kSweepBlocks = 2;  // per multiprocessor
+constexpr int kSpareMax = 32 * 8;  // per lane: 8 released but one it keeps, and a queue entry
+
+// the first frontier's cells, as queue entries
+__global__ void k_drain_seed(const uint32_t* __restrict__ front, DrainSync* g,
+                             unsigned long long* queue) {
+  const unsigned n = g->tail;
+  for (unsigned k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x)
+    queue[k] = (1ull << 32) | front[k];
+}
+
+__device__ __forceinline__ unsigned long long ld_relaxed(const void* p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+// Predicated forms, without a branch around each: a lane's loads (or atomics)
+// are issued one behind the other and their latencies overlap.
+__device__ __forceinline__ unsigned long long ld_relaxed_if(bool on, const void* p) {
+  unsigned long long v;
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.u32 p, %2, 0;\n mov.u64 %0, 0;\n"
+      " @p ld.relaxed.gpu.global.u64 %0, [%1];\n}"
+      : "=l"(v)
+      : "l"(p), "r"((unsigned)on)
+      : "memory");
+  return v;
+}
+__device__ __forceinline__ unsigned long long ld_const_if(bool on, const void* p) {
+  unsigned long long v;
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.u32 p, %2, 0;\n mov.u64 %0, 0;\n"
+      " @p ld.global.nc.u64 %0, [%1];\n}"
+      : "=l"(v)
+      : "l"(p), "r"((unsigned)on));
+  return v;
+}
+__device__ __forceinline__ int count_down_if(bool on, int* p) {  // the old count, 0 when off
+  int v;
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.u32 p, %2, 0;\n mov.u32 %0, 0;\n"
+      " @p atom.relaxed.gpu.global.add.s32 %0, [%1], -1;\n}"
+      : "=r"(v)
+      : "l"(p), "r"((unsigned)on)
+      : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_relaxed(void* p, unsigned long long v) {
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+
+// The accumulation, without frontiers or barriers: a lane sums a ready cell,
+// stores its area, counts down its lower neighbours and goes on with one that
+// this made ready; the others go to a queue, from which lanes without a cell
+// take theirs in turn.  The areas themselves tell when they are there (a NaN
+// until then), so no fence stands between a cell's sum and its neighbours'
+// counts; a lane that was handed a cell before the last area arrived asks
+// again.  Lanes never wait for a block that is not running: an entry's lane
+// took its number while it ran.
+//
+// What bounds it is the longest path down the terrain (2,000 to 3,200 cells
+// at 1024^2 to 2000^2) times one cell's latency.  A cell costs two round trips
+// to L2: one for its shares and its neighbours' areas, one for the counts of
+// its lower neighbours, whose heads come along with it, so that the next
+// cell's terms are known when its count is; the loads and atomics of a
+// round trip are predicated instructions in a row (as branches they ran one
+// after the other: 4,300 cycles for the counts instead of 1,400).  The
+// queue's loads are issued with the first round trip and its entries written
+// behind it; cells that a lane releases beyond one go to idle lanes of its
+// warp before the queue.
+// Frontier by frontier (grid barriers, or one block alone on small frontiers)
+// a cell of the path took 9-10 us, now 2 us: 18.1 -> 4.0 ms at 1024^2,
+// 32 -> 7.0 ms at 2000^2.  More or fewer warps than two blocks of 128 per
+// multiprocessor are slower (one: 7.1, four: 7.7 ms at 2000^2).
+__global__ void __launch_bounds__(kSweepThreads) k_drain_sweep(const hc_view c, DrainSync* g,
+                                                               unsigned long long* queue) {
+  const unsigned FULL = 0xffffffffu;
   const unsigned lane = threadIdx.x & 31;
-  for (unsigned k0 = start - lane; k0 < n_in; k0 += stride) {
-    const unsigned k = k0 + lane;
-    uint32_t cell = 0;
-    unsigned rel = 0;
-    if (k < n_in) {
-      cell = __ldcg(&fin[k]);
-      rel = drain_cell_g(c, el, cell);
-    }
-    const unsigned cnt = __popc(rel);
-    unsigned incl = cnt;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += y;
-    }
-    unsigned base = 0;
-    if (lane == 31 && incl) base = atomicAdd(n_out, incl);
-    base = __shfl_sync(0xffffffffu, base, 31);
-    unsigned m = base + incl - cnt;
-    const int W = (int)c.W;
-    while (rel) {
-      const int kk = __ffs(rel) - 1;
-      rel &= rel - 1;
-      __stcg(&fout[m++], (uint32_t)((int)cell + (kk / 3 - 1) * W + (kk % 3 - 1)));
-    }
-  }
-}
-
-// All frontiers in one cooperative launch, one grid barrier between
-// frontiers, or block 0 alone while they are small.  Each cell enters
-// exactly one frontier, so at most imax*jmax cells are processed.
-__global__ void __launch_bounds__(512, 1) k_drain_sweep(const hc_view c, hc_dev* d,
-                                                      const double* __restrict__ el,
-                                                      DrainSync* g) {
-  __shared__ unsigned s_cnt;
-  __shared__ bool s_ok;
-  const unsigned nblocks = gridDim.x;
-  const unsigned gtid = blockIdx.x * blockDim.x + threadIdx.x;
-  const unsigned gsize = nblocks * blockDim.x;
-  const unsigned long long M = (unsigned long long)c.imax * c.jmax;
-  // the waits' limits (a test may shorten them and make the barrier
-  // expect more arrivals than there are blocks)
-  const bool test = c.wait_spins > 0;
-  const long bar_limit = test ? (long)c.wait_spins : (1L << 22);
-  const long solo_limit = test ? (long)c.wait_spins : (1L << 24);
-  const unsigned expect = nblocks + (test ? (unsigned)c.barrier_extra : 0u);
-  const unsigned solo_max = (test && c.barrier_extra > 0) ? 0u : kSoloMax;
-  unsigned long long done = 0;
-  unsigned level = 0;
-  uint32_t* fr[2] = {c.drain_f0, c.drain_f1};
+  const int W = (int)c.W;
+  const bool test = c.wait_spins > 0;  // a test shortens the waits and has them run out
+  const long limit = test ? (long)c.wait_spins : (1L << 24);
+  const unsigned long long M =
+      (unsigned long long)c.imax * c.jmax + (test ? (unsigned)c.barrier_extra : 0u);
+  uint32_t cell = 0;             // 0: none (cell 0 is a padding cell)
+  unsigned long long head = 0;   // of `cell`
+  unsigned hop = 0, most = 0;
+  unsigned slot = 0;
+  bool ticket = false;           // the lane waits for queue entry `slot`
+  unsigned finished = 0;         // cells finished by the lane since the last report
+  long idle = 0;
+  __shared__ uint4 spare[kSweepThreads / 32][kSpareMax];  // released: cell, hop, head
+  uint4* mine = spare[threadIdx.x >> 5];
+  unsigned out0 = 0, out1 = 0;   // of them, [out0, out1) go to the queue ...
+  unsigned base = 0;             // ... at this place (lane 0)
   for (;;) {
-    const unsigned cur = level % 3, nxt = (level + 1) % 3;
-    const unsigned n_in = *(volatile unsigned*)&g->count[cur];
-    if (n_in == 0 || *(volatile unsigned*)&g->err) break;
-    if (n_in <= solo_max) {
-      if (blockIdx.x == 0) {
-        unsigned n = n_in;
-        for (;;) {
-          if (threadIdx.x == 0) s_cnt = 0;
-          __syncthreads();
-          drain_frontier(c, el, fr[level & 1], n, fr[(level + 1) & 1], &s_cnt, threadIdx.x,
-                         blockDim.x);
-          __syncthreads();
-          const unsigned nn = s_cnt;
-          __syncthreads();  // all have read s_cnt before it is cleared
-          done += n;
-          level++;
-          n = nn;
-          if (done > M) {  // cannot happen: "higher than" has no cycles
-            if (threadIdx.x == 0) atomicExch(&g->err, 2u);
-            break;
-          }
-          if (n == 0 || n > solo_max) break;
-        }
-        if (threadIdx.x == 0) {
-          g->count[level % 3] = n;
-          g->count[(level + 1) % 3] = 0;
-          g->solo_done = done;
-          __threadfence();
-          atomicExch(&g->solo_level, level);  // the other blocks go on from here
-        }
-        __syncthreads();
-      } else {
-        if (threadIdx.x == 0) {
-          s_ok = true;
-          long spins = 0;
-          while (*(volatile unsigned*)&g->solo_level <= level) {
-            if (++spins > solo_limit || *(volatile unsigned*)&g->err) {
-              atomicExch(&g->err, 1u);
-              s_ok = false;
-              break;
-            }
-            __nanosleep(256);
-          }
-          __threadfence();
-        }
-        __syncthreads();
-        if (!s_ok) break;
-        level = *(volatile unsigned*)&g->solo_level;
-        done = *(volatile unsigned long long*)&g->solo_done;
-      }
-      continue;
+    // first round trip: the cell's terms, or the lane's queue entry
+    const int n = cell != 0 ? (int)(head >> kHeadCount) & 15 : 0;
+    const double* share = c.drain_share + (size_t)cell * 8;
+    unsigned long long s[8], a[8];
+#pragma unroll
+    for (int t = 0; t < 8; t++) {
+      const int k = (int)(head >> (4 * t)) & 15;
+      s[t] = ld_const_if(t < n, share + t);
+      a[t] = ld_relaxed_if(t < n, c.area + ((int)cell + (k / 3 - 1) * W + k % 3 - 1));
     }
-    drain_frontier(c, el, fr[level & 1], n_in, fr[(level + 1) & 1], &g->count[nxt], gtid, gsize);
-    if (gtid == 0) g->count[(level + 2) % 3] = 0;  // read two frontiers ago
-    done += n_in;
-    level++;
-    if (done > M) {  // cannot happen: "higher than" has no cycles
-      if (gtid == 0) atomicExch(&g->err, 2u);
+    const unsigned long long q = ld_relaxed_if(ticket && slot < (unsigned)c.N2, queue + slot);
+    // the last turn's released cells, at the place their atomic gave
+    if (out1 > out0) {
+      const unsigned m = __shfl_sync(FULL, base, 0);
+      for (unsigned k = out0 + lane; k < out1; k += 32)
+        st_relaxed(queue + m + (k - out0),
+                   ((unsigned long long)mine[k].y << 32) | mine[k].x);
+      __syncwarp();
+      out1 = out0 = 0;
+    }
+    bool ready = cell != 0;
+#pragma unroll
+    for (int t = 0; t < 8; t++) ready = ready && a[t] != ~0ull;
+    const int n_warp = (int)__reduce_max_sync(FULL, (unsigned)n);
+    uint32_t next = ready ? 0u : cell;
+    unsigned long long next_head = head;
+    unsigned next_hop = hop, rel = 0;
+    unsigned long long hd[9];
+    if (ready) {
+      double sum = ((head >> kHeadOwn) & 1u) ? 1.0 : 0.0;
+#pragma unroll
+      for (int t = 0; t < 8; t++)  // the terms past n are +0, which adds nothing
+        if (t < n_warp)
+          sum += __longlong_as_double((long long)a[t]) * __longlong_as_double((long long)s[t]);
+      if (!((head >> kHeadReached) & 1u) || !(sum > 0)) sum = 0;
+      st_relaxed(c.area + cell, (unsigned long long)dbits(sum));
+      // second round trip: the lower neighbours' counts and heads
+      const unsigned lower = (unsigned)(head >> kHeadLower) & 0x1ffu;
+      int old[9];
+#pragma unroll
+      for (int k = 0; k < 9; k++) {
+        const int nb = (int)cell + (k / 3 - 1) * W + k % 3 - 1;
+        const bool low = k != 4 && ((lower >> k) & 1u);
+        old[k] = count_down_if(low, &c.drain_pend[nb]);
+        hd[k] = ld_const_if(low, c.drain_head + nb);
+      }
+#pragma unroll
+      for (int k = 8; k >= 0; k--)
+        if (old[k] == 1) {
+          rel |= 1u << k;
+          next = (uint32_t)((int)cell + (k / 3 - 1) * W + k % 3 - 1);
+          next_head = hd[k];
+        }
+      rel &= rel - 1;  // the lane goes on with the lowest of them itself
+      next_hop = hop + 1;
+      finished++;
+      most = max(most, hop);
+    } else if (cell != 0) {
+      idle++;  // an area still on its way
+    }
+    // the lane's queue entry: its own when it is idle (it may have been given
+    // a cell by another lane since it took its number), else one more to share
+    bool extra = false;
+    unsigned long long q_head = 0;
+    if (q) {
+      q_head = __ldg(c.drain_head + (uint32_t)q);
+      ticket = false;
+      if (next == 0) {
+        next = (uint32_t)q;
+        next_hop = (unsigned)(q >> 32);
+        next_head = q_head;
+      } else {
+        extra = true;
+      }
+    }
+    const unsigned cnt = __popc(rel) + (extra ? 1u : 0u);
+    if (__any_sync(FULL, cnt != 0)) {
+      // cells beyond one per lane: to the warp's idle lanes first (a cell that
+      // goes by the queue loses two more round trips), the rest to the queue
+      unsigned incl = cnt;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned y = __shfl_up_sync(FULL, incl, o);
+        if (lane >= (unsigned)o) incl += y;
+      }
+      const unsigned total = __shfl_sync(FULL, incl, 31);
+      unsigned m = incl - cnt;
+#pragma unroll
+      for (int k = 0; k < 9; k++)
+        if ((rel >> k) & 1u)
+          mine[m++] = make_uint4((unsigned)((int)cell + (k / 3 - 1) * W + k % 3 - 1), hop + 1,
+                                 (unsigned)hd[k], (unsigned)(hd[k] >> 32));
+      if (extra)
+        mine[m] = make_uint4((unsigned)q, (unsigned)(q >> 32), (unsigned)q_head,
+                             (unsigned)(q_head >> 32));
+      __syncwarp();
+      const unsigned free = __ballot_sync(FULL, next == 0);
+      const unsigned take = min(total, (unsigned)__popc(free));
+      const unsigned r = __popc(free & ((1u << lane) - 1u));
+      if (next == 0 && r < take) {
+        const uint4 e = mine[r];
+        next = e.x;
+        next_hop = e.y;
+        next_head = ((unsigned long long)e.w << 32) | e.z;
+      }
+      out0 = take;
+      out1 = total;
+      if (lane == 0 && total > take) base = atomicAdd(&g->tail, total - take);
+    }
+    cell = next;
+    head = next_head;
+    hop = next_hop;
+    // a queue number for each lane that needs one, one atomic per warp
+    const unsigned want = __ballot_sync(FULL, cell == 0 && !ticket);
+    if (want) {
+      unsigned first = 0;
+      const int leader = __ffs(want) - 1;
+      if ((int)lane == leader) first = atomicAdd(&g->taken, (unsigned)__popc(want));
+      first = __shfl_sync(FULL, first, leader);
+      if ((want >> lane) & 1u) {
+        slot = first + __popc(want & ((1u << lane) - 1u));
+        ticket = true;
+      }
+    }
+    if (out1 == out0 && !__any_sync(FULL, cell != 0)) {
+      // nothing to do: report, and leave when every cell is finished
+      unsigned f = finished;
+      for (int o = 16; o > 0; o >>= 1) f += __shfl_xor_sync(FULL, f, o);
+      finished = 0;
+      unsigned stop = 0;
+      if (lane == 0) {
+        if (f) atomicAdd(&g->done, (unsigned long long)f);
+        if (ld_relaxed(&g->done) >= M) {
+          stop = 1;
+        } else if (++idle > limit || *(volatile unsigned*)&g->err) {
+          atomicExch(&g->err, 1u);
+          stop = 1;
+        } else {
+          __nanosleep(64);
+        }
+      }
+      if (__shfl_sync(FULL, stop, 0)) break;
+    }
+    if (__any_sync(FULL, idle > limit)) {
+      if (lane == 0) atomicExch(&g->err, 1u);
       break;
     }
-    if (!grid_barrier(g, expect, bar_limit)) break;
   }
-  if (gtid == 0) {
-    d->drain_done = (unsigned)done;
-    d->drain_levels = level;
-    d->drain_front = 0;
-    if (g->err) {
-      d->err_code = 401;
-      d->pause |= HC_PAUSE_ERROR;
-    }
+  for (int o = 16; o > 0; o >>= 1) most = max(most, __shfl_xor_sync(FULL, most, o));
+  if (lane == 0) atomicMax(&g->hops, most);
+}
+
+// the sweep's outcome into the control block
+__global__ void k_drain_end(hc_dev* d, const DrainSync* g) {
+  d->drain_done = (unsigned)g->done;
+  d->drain_levels = g->hops;
+  d->drain_front = 0;
+  if (g->err) {
+    d->err_code = 401;
+    d->pause |= HC_PAUSE_ERROR;
   }
 }
 
@@ -628,8 +659,7 @@ hc_status run_drainage_device(hc_ctx* c, const double* el, bool area_valid,
       k_sel_pick<<<1, 1, 0, s>>>(v, shift, P);
     }
     k_drain_init<<<g, b, 0, s>>>(v, c->dev, el);
-    k_drain_frac<<<g, b, 0, s>>>(v, el);
-    c->launches += 20;
+    c->launches += 19;
     hc_drain_aux a;
     if (cudaMemcpyAsync(&a, v.drain_aux, sizeof a, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
         cudaStreamSynchronize(s) != cudaSuccess)
@@ -645,39 +675,29 @@ hc_status run_drainage_device(hc_ctx* c, const double* el, bool area_valid,
       c->launches += 1;
       *sorted = true;
     }
-    // the sweep: all blocks resident (cooperative launch), grid barriers
-    // between frontiers
-    int dev = 0, sms = 0, per_sm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    // one block per SM: fewer arrivals at each barrier; a frontier averages a
-    // few thousand cells
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_drain_sweep, 512, 0);
-    const int nblocks = std::max(1, sms * std::min(per_sm, 1));
-    // the barrier lives in the selection's histogram, which is finished
-    static_assert(sizeof(DrainSync) <= sizeof(hc_drain_aux::hist), "barrier fits");
+    k_drain_terms<<<g, b, 0, s>>>(v, el);
+    // the queue takes the place of difftot, which only the terms needed; the
+    // sweep's state that of the selection's histogram, which is finished
+    static_assert(sizeof(DrainSync) <= sizeof(hc_drain_aux::hist), "sweep state fits");
     DrainSync* gs = (DrainSync*)((char*)v.drain_aux + offsetof(hc_drain_aux, hist));
+    unsigned long long* queue = (unsigned long long*)v.drain_dt;
     const unsigned* front = (const unsigned*)((const char*)c->dev + offsetof(hc_dev, drain_front));
     if (cudaMemsetAsync(gs, 0, sizeof(DrainSync), s) != cudaSuccess ||
-        cudaMemcpyAsync((char*)gs + offsetof(DrainSync, count), front, sizeof(unsigned),
+        cudaMemsetAsync(queue, 0, N2 * 8, s) != cudaSuccess ||
+        cudaMemcpyAsync((char*)gs + offsetof(DrainSync, tail), front, sizeof(unsigned),
                         cudaMemcpyDeviceToDevice, s) != cudaSuccess)
       return HC_ERR_CUDA;
+    k_drain_seed<<<c->sms, 256, 0, s>>>(v.drain_f0, gs, queue);
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     cudaEventRecord(e0, s);
-    const double* elp = el;
-    hc_dev* devp = c->dev;
-    void* args[] = {(void*)&v, (void*)&devp, (void*)&elp, (void*)&gs};
-    const cudaError_t le = cudaLaunchCooperativeKernel((const void*)k_drain_sweep, nblocks, 512,
-                                                       args, 0, s);
+    const int nblocks = (int)std::max<size_t>(
+        1, std::min<size_t>((size_t)c->sms * kSweepBlocks, (M + 1023) / 1024));
+    k_drain_sweep<<<nblocks, kSweepThreads, 0, s>>>(v, gs, queue);
     cudaEventRecord(e1, s);
-    c->launches += 1;
-    if (le != cudaSuccess) {
-      cudaEventDestroy(e0);
-      cudaEventDestroy(e1);
-      return HC_ERR_CUDA;
-    }
+    k_drain_end<<<1, 1, 0, s>>>(c->dev, gs);
+    c->launches += 4;
     if (cudaEventSynchronize(e1) == cudaSuccess) {
       float ms = 0;
       cudaEventElapsedTime(&ms, e0, e1);

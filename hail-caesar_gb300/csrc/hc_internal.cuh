@@ -178,13 +178,14 @@ struct hc_view {
   double *pre;                   // 12 * N2: per-cell apply-pass terms, side by side (PRE)
   uint32_t *chains;              // 4 * N2: apply-pass chain starts (x pass, y pass), then
                                  // the resume points of long chains (x, y)
-  // drainage area (hc_drain.cu): sweep position, sum of drops, higher
-  // neighbours pending, two frontiers, and the elevation snapshot
+  // drainage area (hc_drain.cu): sweep position, sum of drops (then the
+  // sweep's queue), higher neighbours pending, the first frontier, the sort's
+  // order, and the elevation snapshot
   uint32_t *drain_pos, *drain_f0, *drain_f1;
   int32_t *drain_pend;
   double *drain_dt, *drain_snap;
-  double *drain_frac;     // 9*N2: share of neighbour k's area pushed here (plane k)
-  uint16_t *drain_multi;  // N2: neighbours (bit k) that push here in more than one direction
+  double *drain_share;    // 8*N2: a cell's shares of its higher neighbours' areas, in sweep order
+  unsigned long long *drain_head;  // N2: which neighbours they are, and the lower ones
   struct hc_drain_aux *drain_aux;
   // adjoint runs (hc_adjoint.cu): per-iteration time steps, recorded or
   // imposed (HC_ADJ_REC stride per iteration; see hc_dev::adj_mode)

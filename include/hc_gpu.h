@@ -372,7 +372,7 @@ enum {
   HC_STAT_DRAINAGE,        /* drainage area + input points (baseflow change) */
   HC_STAT_DRAINAGE_SORT,   /* of those, sorts of the elevations (equal elevations that matter) */
   HC_STAT_DRAINAGE_SWEEP,  /* device accumulation (ms: device time) */
-  HC_STAT_DRAINAGE_LEVELS, /* frontiers the accumulations went through (count) */
+  HC_STAT_DRAINAGE_LEVELS, /* cells on the accumulations' longest chains of releases (count) */
   HC_STAT_IDLE_ITERS,      /* captured iterations skipped after a pause */
   HC_STAT_DRAINAGE_HOST_SORT, /* of the sorts, those the host finished (see hc_drainage_sort) */
   HC_STAT_WET_CELL_STEPS,  /* count: wet-list cells summed over the iterations run (the
