@@ -942,97 +942,163 @@ __global__ void __launch_bounds__(1024) k_wet_write(const hc_view c, const hc_de
 }
 
 // ---------------------------------------------------------------------------
-// water_flux_out :3005-3047, one block.  Each edge cell is clamped at its
-// first visit in the reference's loop order; the outflow sum is a fixed-order
-// tree (deterministic, equal to the serial sum up to rounding).
+// water_flux_out :3005-3047.  Each edge cell is clamped at its first visit in
+// the reference's loop order; the outflow sum is a fixed-order tree
+// (deterministic, equal to the serial sum up to rounding).
 // Also writes the iteration record and the end-of-loop test of main.cpp:204.
+//
+// The blocks clamp the cells and leave each one's outflow and depth in
+// c.flux; the block that finishes last adds them.  One block did it all
+// before, and the cells' FP64 operations (a division among them) waited for
+// one multiprocessor's FP64 pipe (ncu, cold caches: 23 -> 12 us at 1024^2,
+// 30 -> 15 us at 1400^2).  The sum's order is that of the
+// one block of 1024 threads (thread t: t, t + 1024, ...; then the tree).
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(1024) k_flux_out(const hc_view c, hc_dev* d, int gated, int record,
-                                                    hc_step_record* rec, int64_t rec_cap) {
-  __shared__ double part[1024];
-  __shared__ double vpart[1024];
+constexpr int kFluxSums = 1024, kFluxThreads = 512;
+
+__global__ void __launch_bounds__(kFluxThreads) k_flux_out(const hc_view c, hc_dev* d, int gated, int record,
+                                                   hc_step_record* rec, int64_t rec_cap) {
+  __shared__ double part[kFluxSums];
+  __shared__ double vpart[kFluxSums];
   if (gated && !(d->it_active && d->rest_active)) return;
   const hc_params& p = c.p;
   const int imax = c.imax, jmax = c.jmax;
   const double thr = p.water_depth_erosion_threshold, DX = p.DX;
-  const double fdt = d->s.time_step;
+  const hc_divisor fdt = ddiv_prep(d->s.time_step);
   const int n1 = 2 * imax, n2 = n1 + 2 * jmax;
-  double acc = 0, vacc = 0;  // the outflow rate, and the depth taken off
-  for (int k = threadIdx.x; k < n2; k += blockDim.x) {
+  const bool solo = gridDim.x == 1;
+  double* rates = c.flux;      // the outflow rate per edge cell
+  double* depths = c.flux + n2;  // and the depth taken off
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n2; k += gridDim.x * blockDim.x) {
     int i, j;
+    bool first = true;
     if (k < n1) {
       i = 1 + k / 2;
       if ((k & 1) == 0) {
         j = jmax;
       } else {
         j = 1;
-        if (jmax == 1) continue;  // same cell as the right-hand edge
+        if (jmax == 1) first = false;  // same cell as the right-hand edge
       }
     } else {
       const int kk = k - n1;
       j = 1 + kk / 2;
-      if (j == 1 || j == jmax) continue;  // already visited by the row loop
+      if (j == 1 || j == jmax) first = false;  // already visited by the row loop
       if ((kk & 1) == 0) {
         i = 1;
       } else {
         i = imax;
-        if (imax == 1) continue;
+        if (imax == 1) first = false;
       }
     }
-    double& h = c.h[(size_t)i * c.W + j];
-    if (h > thr) {
-      acc += (h - thr) * DX * DX / fdt;
-      vacc += h - thr;
-      h = thr;
+    double rate = 0, off = 0;
+    if (first) {
+      double& h = c.h[(size_t)i * c.W + j];
+      const double h0 = h;
+      if (h0 > thr) {
+        off = h0 - thr;
+        rate = ddiv_by(off * DX * DX, fdt);
+        h = thr;
+      }
+    }
+    if (solo) {  // at most kFluxSums cells: each is a sum of its own
+      part[k] = rate;
+      vpart[k] = off;
+    } else {
+      rates[k] = rate;
+      depths[k] = off;
     }
   }
-  part[threadIdx.x] = acc;
-  vpart[threadIdx.x] = vacc;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w) {
-      part[threadIdx.x] += part[threadIdx.x + w];
-      vpart[threadIdx.x] += vpart[threadIdx.x + w];
+  if (!solo && !last_to_arrive(&d->flux_arrive)) return;
+  // what the record takes, on its way while the sums are formed
+  hc_scalars& s = d->s;
+  hc_step_record r;
+  double vin = 0, vlost = 0, vmask = 0, vin_tot = 0, vout_tot = 0, vlost_tot = 0, vmask_tot = 0;
+  double vol = 0, vol_counter = 0, creep1 = 0, creep2 = 0;
+  if (threadIdx.x == 0) {
+    r.counter = s.counter;
+    r.cycle = s.cycle;
+    r.time_step = s.time_step;
+    r.maxdepth = d->maxdepth_step;
+    r.waterinput = s.waterinput;
+    r.erode_mult = s.erode_mult;
+    r.sediQ = s.sediQ;
+    r.globalsediq = s.globalsediq;
+    r.baseflow = s.baseflow;
+    creep1 = s.creep_time;
+    creep2 = s.creep_time2;
+    vin = d->vin_step;
+    vlost = d->vlost_step;
+    vmask = d->vmask_step;
+    vin_tot = d->vin_tot;
+    vout_tot = d->vout_tot;
+    vlost_tot = d->vlost_tot;
+    vmask_tot = d->vmask_tot;
+    vol = d->vol_scan;
+    vol_counter = d->vol_scan_counter;
+  }
+  // nothing flowed off a cell whose entry is zero (rates and depths are never
+  // negative, so leaving a +0 out changes no sum)
+  for (int t = threadIdx.x; t < kFluxSums; t += blockDim.x) {
+    if (solo) {
+      if (t >= n2) part[t] = vpart[t] = 0;
+      continue;
     }
-    __syncthreads();
+    double acc = 0, vacc = 0;
+    for (int k0 = t; k0 < n2; k0 += 4 * kFluxSums) {
+      double rt[4], of[4];
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        const int k = k0 + q * kFluxSums;
+        of[q] = k < n2 ? __ldcg(depths + k) : 0.0;
+        rt[q] = k < n2 ? __ldcg(rates + k) : 0.0;
+      }
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+        if (dbits(of[q]) != 0) {
+          acc += rt[q];
+          vacc += of[q];
+        }
+    }
+    part[t] = acc;
+    vpart[t] = vacc;
+  }
+  __syncthreads();
+  for (int w = kFluxSums / 2; w > 0; w >>= 1) {
+    for (int t = threadIdx.x; t < w; t += blockDim.x)
+      if (dbits(vpart[t + w]) != 0) {
+        part[t] += part[t + w];
+        vpart[t] += vpart[t + w];
+      }
+    if (w > 32) __syncthreads();
+    else __syncwarp();
   }
   if (threadIdx.x == 0) {
-    hc_scalars& s = d->s;
     s.temptot = part[0];
-    s.waterOut = s.temptot;
+    s.waterOut = part[0];
     if (record && rec && d->rec_index < rec_cap) {
-      hc_step_record& r = rec[d->rec_index];
-      r.counter = s.counter;
-      r.cycle = s.cycle;
-      r.time_step = s.time_step;
-      r.maxdepth = d->maxdepth_step;
-      r.waterOut = s.waterOut;
-      r.waterinput = s.waterinput;
-      r.erode_mult = s.erode_mult;
-      r.sediQ = s.sediQ;
-      r.globalsediq = s.globalsediq;
-      r.baseflow = s.baseflow;
+      r.waterOut = part[0];
       const double a2 = DX * DX;
-      r.vol_in = d->vin_step * a2;
-      r.vol_out = (vpart[0] + d->vlost_step) * a2;
-      r.vol_mask = d->vmask_step * a2;
-      r.volume = (d->vol_scan_counter == s.counter) ? d->vol_scan * a2 : __longlong_as_double(0x7ff8000000000000LL);
+      r.vol_in = vin * a2;
+      r.vol_out = (vpart[0] + vlost) * a2;
+      r.vol_mask = vmask * a2;
+      r.volume = (vol_counter == r.counter) ? vol * a2 : __longlong_as_double(0x7ff8000000000000LL);
+      rec[d->rec_index] = r;
     }
     if (record) d->rec_index++;
     if (gated) d->wet_steps += (unsigned long long)d->wet_count;
     // the ledger: this iteration's terms join the totals
-    d->vin_tot += d->vin_step;
-    d->vout_tot += vpart[0];
-    d->vlost_tot += d->vlost_step;
-    d->vmask_tot += d->vmask_step;
+    d->vin_tot = vin_tot + vin;
+    d->vout_tot = vout_tot + vpart[0];
+    d->vlost_tot = vlost_tot + vlost;
+    d->vmask_tot = vmask_tot + vmask;
     d->vin_step = 0;
     d->vlost_step = 0;
     d->vmask_step = 0;
     if (gated) {
-      if (!p.hydro_only && !(d->flags & HC_RUN_NOHILL) &&
-          (s.cycle > s.creep_time || s.cycle > s.creep_time2))
+      if (!p.hydro_only && !(d->flags & HC_RUN_NOHILL) && (r.cycle > creep1 || r.cycle > creep2))
         d->pause |= HC_PAUSE_HOSTSTEP;
-      if (!(s.cycle / 60 < p.maxcycle)) d->pause |= HC_PAUSE_FINISHED;
+      if (!(r.cycle / 60 < p.maxcycle)) d->pause |= HC_PAUSE_FINISHED;
     }
   }
 }
@@ -1170,7 +1236,12 @@ static void wet_list(hc_ctx* c, int gated, int nvol) {
 }
 
 void launch_flux_out(hc_ctx* c, int gated, int record) {
-  k_flux_out<<<1, 1024, 0, c->cs>>>(c->v, c->dev, gated, record, c->v.rec, c->v.rec_cap);
+  const int n = 2 * (c->v.imax + c->v.jmax);
+  // one block while every cell can be a sum of its own: nothing goes through
+  // memory then, and no block waits for another's arrival
+  const int blocks = n <= kFluxSums ? 1 : std::min((n + kFluxThreads - 1) / kFluxThreads, 64);
+  k_flux_out<<<blocks, kFluxThreads, 0, c->cs>>>(c->v, c->dev, gated, record, c->v.rec,
+                                                 c->v.rec_cap);
   count_launch(c, 1);
 }
 

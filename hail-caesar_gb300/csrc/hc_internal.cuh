@@ -80,8 +80,8 @@ struct hc_dev {
   unsigned int misc_done;
   // arrival counters of the launches whose last block finishes the step
   // (last_to_arrive): the wet list's count, the grain records' count and
-  // assignment, slide_3's flag count; each is zero between launches
-  unsigned int wet_arrive, alloc_arrive, assign_arrive, flag_arrive;
+  // assignment, slide_3's flag count, the edge outflow; each is zero between launches
+  unsigned int wet_arrive, alloc_arrive, assign_arrive, flag_arrive, flux_arrive;
   unsigned long long body_kernels;  // kernels run inside conditional graph nodes
   int wet_count;          // length of hc_view::wet
   int do_drain;           // this iteration moved the baseflow threshold
@@ -201,6 +201,7 @@ struct hc_view {
   uint8_t *touched;              // N2 bytes
   double *red;                   // reduction scratch
   int32_t *scan_tmp;             // scan scratch
+  double *flux;                  // water_flux_out: 2 * (2 imax + 2 jmax) edge-cell terms
   double *vpart; int vpart_cap;  // per-block partial sums (grid_sum, scan_area's volume)
   hc_step_record *rec; int64_t rec_cap;
   // test hook of the bounded device waits (hc_test_bounded_waits): when
