@@ -32,126 +32,160 @@ __device__ __forceinline__ double flow_dt_of(const hc_params& p, const hc_scalar
 
 // ---------------------------------------------------------------------------
 // control: set_loop_cycle .. catchment_waterinputs (main.cpp:142-158), one
-// thread.  Also decides which members run in this iteration.
+// warp.  Also decides which members run in this iteration.
+//
+// Every lane forms the scalars (the same values) and lane 0 stores them; lane
+// z holds rain zone z, and lane n the grain fraction n + 1 of a reach's
+// sediment input, whose sums run over the lanes in the reference's order.
+// The kernel runs alone, once an iteration, so its time is latency: dependent
+// FP64 operations (divisions on the integer pipe), loads, and the fetch of its
+// instructions, which no other launch has left in the cache.  Hence one copy
+// of each long operation and rolled loops (ncu, cold caches: 65 -> 16 us for a
+// reach, one point and nine fractions, 18 -> 7.3 us without; one thread before).
 // ---------------------------------------------------------------------------
-__device__ void topmodel_step(hc_dev* d, const hc_params& p, const double* topm, int rows) {
-  // topmodel_runoff(time_1) :3649-3715: the recurrence depends only on the
-  // rain table, so the host evaluates it once (host_topmodel_table) and the
-  // device steps through the rows.
-  int t = (int)d->s.time_1;
-  const int rf = p.rfnum;
-  if (t < 0 || t >= rows) {
-    d->err_code = 101;
-    d->pause |= HC_PAUSE_ERROR;
-    return;
-  }
-  const double* row = topm + (size_t)t * 2 * (rf + 1);
-  for (int n = p.spatially_complex_rainfall ? 0 : 1; n <= rf; n++) {
-    d->s.old_j_mean[n] = row[n];
-    d->s.new_j_mean[n] = row[(rf + 1) + n];
-  }
+static __device__ __noinline__ double cdiv(double a, double b) { return ddiv_rn(a, b); }
+static __device__ __noinline__ double csqrt(double x) { return isqrt_rn(x); }
+
+// (long long)x % m for a counter x >= 0, m >= 1
+__device__ __forceinline__ bool divides(double x, int m) {
+  if (x < 2147483647.0) return (unsigned)x % (unsigned)m == 0;
+  return (long long)x % m == 0;
 }
 
-__global__ void k_control(const hc_view c, hc_dev* d, hc_iter_handles hh) {
+// sediment input of a reach point (:3310-3396): the fractions' amounts, one
+// per lane, then the sums in fraction order
+__device__ __noinline__ void reach_sediment(const hc_view& c, hc_dev* d, int n, int row,
+                                            double time_step) {
+  const hc_params& p = c.p;
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const size_t cell = (size_t)p.inpoints[n][0] * c.W + p.inpoints[n][1];
+  if (!(c.h[cell] > p.water_depth_erosion_threshold) || row >= c.reach_rows[n]) return;
+  const int rdt = p.reach_input_data_timestep, div = p.div_inputs;
+  const double a2 = p.DX * p.DX, secs = (double)(rdt * 60);
+  const bool mine = lane < HC_NFRAC;  // fraction lane + 1, column lane + 5
+  const float r = mine ? fabsf(c.reach[n][(size_t)row * c.reach_cols[n] + 5 + lane]) : 0.0f;
+  const float q = r / div;  // float / int in the reference
+  const double part = cdiv(cdiv((double)q, a2), secs) * time_step;
+  double added_tot = 0, adding_factor = 1;
+#pragma unroll 1
+  for (int k = 0; k < HC_NFRAC; k++) added_tot += __shfl_sync(FULL, part, k);
+  if (cdiv(added_tot, (double)p.number_of_points) > p.ERODEFACTOR * 0.75)
+    adding_factor = cdiv(p.ERODEFACTOR * 0.75, cdiv(added_tot, (double)p.number_of_points));
+  if (c.index[cell] == -9999) {  // addGS :3949, serial position: now
+    __syncwarp();
+    if (lane == 0) {
+      d->grain_tot++;
+      c.index[cell] = d->grain_tot;
+      grain_record_init(c, cell, c.elev[cell], c.bed[cell]);
+    }
+    __syncwarp();
+  }
+  const double amt =
+      cdiv(cdiv(cdiv(adding_factor * (double)r, (double)div), a2), secs) * time_step;
+  if (mine && !p.isSuspended[lane + 1]) grain_at(c, cell, lane + 1) += amt;
+  double e = c.elev[cell], vs = c.vs[cell];
+#pragma unroll 1
+  for (int k = 0; k < HC_NFRAC; k++) {
+    const double a = __shfl_sync(FULL, amt, k);
+    if (p.isSuspended[k + 1]) vs += a;
+    else e += a;
+  }
+  __syncwarp();
+  if (lane == 0) {
+    c.elev[cell] = e;
+    c.vs[cell] = vs;
+  }
+  __syncwarp();
+}
+
+__global__ void __launch_bounds__(32) k_control(const hc_view c, hc_dev* d, hc_iter_handles hh) {
   const hc_params& p = c.p;
   hc_scalars& s = d->s;
-  if (d->pause || d->budget <= 0) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const bool l0 = lane == 0;
+  int pause = d->pause;
+  const int64_t budget = d->budget;
+  if (pause || budget <= 0) {
     // skipped iteration: every gated kernel of it returns at once; the
     // switches of the iteration that paused stay as they are, for the host
     // to finish that iteration
-    if (d->budget <= 0) d->pause |= HC_PAUSE_BUDGET;
-    d->it_active = 0;
+    __syncwarp();
+    if (l0) {
+      if (budget <= 0) d->pause = pause | HC_PAUSE_BUDGET;
+      d->it_active = 0;
+    }
     return;
   }
-  d->do_scan = d->do_erode = d->do_slide = d->do_lateral = 0;
-  d->erode_retry = 0;
-  d->erode_passes = 0;
-  d->budget--;
-  d->it_active = 1;
-  d->rest_active = 1;
+  // everything the scalar logic reads, before the first store
+  double time_step = s.time_step, maxdepth = s.maxdepth, cycle = s.cycle, time_1 = s.time_1;
+  double vin = d->vin_step, baseflow = s.baseflow;
+  const double counter = s.counter + 1, erode_call = s.erode_call, erode_mult = s.erode_mult;
+  const double previous = cycle;
+  const double diff = fabs(s.waterinput - s.waterOut);  // set_inputoutput_diff :1879
+  const int rf = p.rfnum;
+  const bool zone = lane <= rf;  // rf <= HC_MAX_RF < 32
+  double jm = zone ? s.j_mean[lane] : 0.0, oldj = zone ? s.old_j_mean[lane] : 0.0,
+         newj = zone ? s.new_j_mean[lane] : 0.0;
+  const double cells = zone ? s.nActualGridCells[lane] : 0.0,
+               points = zone ? s.catchment_input_counter[lane] : 1.0;
+  int err = 0;
 
-  s.previous = s.cycle;                                   // set_loop_cycle :1873
-  s.input_output_difference = fabs(s.waterinput - s.waterOut);  // :1879
-  if (s.maxdepth <= 0.1) s.maxdepth = 0.1;                // set_maximum_timestep :1890
-  if (s.time_step < cfl_dt(p, s.maxdepth)) s.time_step = cfl_dt(p, s.maxdepth);
-  if (s.input_output_difference > p.in_out_difference_allowed &&
-      s.time_step > (cfl_dt(p, s.maxdepth)))
-    s.time_step = cfl_dt(p, s.maxdepth);
+  if (maxdepth <= 0.1) maxdepth = 0.1;                    // set_maximum_timestep :1890
+  // courant_friedrichs_lewy_condition :1884: the depth does not change here
+  const double cfl = p.courant_number * cdiv(p.DX, csqrt(kG * maxdepth));
+  if (time_step < cfl) time_step = cfl;
+  if (diff > p.in_out_difference_allowed && time_step > cfl) time_step = cfl;
   // adjoint runs record the time steps, or impose recorded ones
   const bool adj = c.adj_dt && d->adj_mode && d->adj_i < d->adj_n;
+  const bool impose = adj && d->adj_mode == 2;
   double* arec = adj ? c.adj_dt + (size_t)d->adj_i * HC_ADJ_REC : nullptr;
-  if (adj) {
-    if (d->adj_mode == 2) s.time_step = arec[0];
-    else arec[0] = s.time_step;
-  }
-  s.counter += 1;                                         // increment_counters :1925
-  s.cycle += s.time_step / 60;
+  if (impose) time_step = arec[0];
+  else if (adj && l0) arec[0] = time_step;
+  cycle += cdiv(time_step, 60.0);                         // increment_counters :1925
+  // get_flow_timestep :1913-1923
+  const double fdt = time_step > cfl ? cfl : time_step;
 
   const double DX = p.DX;
   // reach_water_and_sediment_input :3301-3452
   if (p.reach_mode) {
-    const double fdt = flow_dt_of(p, s);
     const int rdt = p.reach_input_data_timestep;
-    const int div = p.div_inputs;
-    const int row = (int)(s.cycle / rdt);
-    if (!p.hydro_only) {
-      for (int n = 0; n <= p.number_of_points - 1; n++) {
-        const int x = p.inpoints[n][0], y = p.inpoints[n][1];
-        const size_t cell = (size_t)x * c.W + y;
-        double adding_factor = 1, added_tot = 0;
-        if (c.h[cell] > p.water_depth_erosion_threshold) {
-          const float* r = c.reach[n] + (size_t)row * c.reach_cols[n];
-          for (int tn = 5; tn <= HC_G + 3; tn++) {
-            float q = fabsf(r[tn]) / div;  // float / int in the reference
-            added_tot += q / (DX * DX) / (rdt * 60) * s.time_step;
-          }
-          if (added_tot / p.number_of_points > p.ERODEFACTOR * 0.75)
-            adding_factor = (p.ERODEFACTOR * 0.75) / (added_tot / p.number_of_points);
-          if (c.index[cell] == -9999) {  // addGS :3949, serial position: now
-            d->grain_tot++;
-            c.index[cell] = d->grain_tot;
-            grain_record_init(c, cell, c.elev[cell], c.bed[cell]);
-          }
-          for (int tn = 5; tn <= HC_G + 3; tn++) {
-            double amt = adding_factor * (double)fabsf(r[tn]) / div / (DX * DX) / (rdt * 60) *
-                         s.time_step;
-            if (p.isSuspended[tn - 4]) {
-              c.vs[cell] += amt;
-            } else {
-              grain_at(c, cell, tn - 4) += amt;
-              c.elev[cell] += amt;
-            }
-          }
-        }
-      }
-    }
+    const int row = (int)cdiv(cycle, (double)rdt);
+    if (!p.hydro_only)
+#pragma unroll 1
+      for (int n = 0; n <= p.number_of_points - 1; n++) reach_sediment(c, d, n, row, time_step);
+#pragma unroll 1
     for (int n = 0; n <= p.number_of_points - 1; n++) {
       const int x = p.inpoints[n][0], y = p.inpoints[n][1];
       const size_t cell = (size_t)x * c.W + y;
       if (row + 1 >= c.reach_rows[n]) {
-        d->err_code = 102;
-        d->pause |= HC_PAUSE_ERROR;
+        err = 102;
+        pause |= HC_PAUSE_ERROR;
         continue;
       }
       double i1 = c.reach[n][(size_t)row * c.reach_cols[n] + 1];
       double i2 = c.reach[n][(size_t)(row + 1) * c.reach_cols[n] + 1];
-      double prop = (((row + 1) * rdt) - s.cycle) / rdt;
+      double prop = cdiv(((row + 1) * rdt) - cycle, (double)rdt);
       double input = i1 + ((i2 - i1) * (1 - prop));
-      s.waterinput += (input / div);
-      const double add = (input / div) / (DX * DX) * fdt;
-      c.h[cell] += add;
-      if (x >= 1 && x <= c.imax && y >= 1 && y <= c.jmax) d->vin_step += add;
+      const double add = cdiv(cdiv(input, (double)p.div_inputs), DX * DX) * fdt;
+      const double h = c.h[cell] + add;
+      __syncwarp();
+      if (l0) c.h[cell] = h;
+      __syncwarp();
+      if (x >= 1 && x <= c.imax && y >= 1 && y <= c.jmax) vin += add;
     }
   }
 
   // catchment_waterinputs :2027 -> catchment_water_input_and_hydrology :3455
-  s.waterinput = 0;
-  double fdt2 = flow_dt_of(p, s);
-  if (adj) {
-    if (d->adj_mode == 2) fdt2 = arec[1];
-    else arec[1] = fdt2;
-  }
-  if (p.spatially_complex_rainfall) {
+  double waterinput = 0, fdt2 = fdt;
+  if (impose) fdt2 = arec[1];
+  else if (adj && l0) arec[1] = fdt2;
+  const bool grid = p.spatially_complex_rainfall != 0;
+  const int z0 = grid ? 0 : 1;  // the first zone that takes part
+  if (zone) d->j_mean_in[lane] = jm;
+  double amt, jmm = 0;
+  if (grid) {
     // catchment_water_input_and_hydrology(flow_timestep, runoff) :3544-3607.
     // A cell's runoff recurrence (runoffGrid::calculate_runoff) depends only
     // on its rain, i.e. on its rain state: the zone (zones 1 .. rfnum-1, or
@@ -159,84 +193,85 @@ __global__ void k_control(const hc_view c, hc_dev* d, hc_iter_handles hh) {
     // and others get no rain, rainGrid::create, LSDRainfallRunoff.cpp:33-66),
     // so every cell of a state holds the
     // same values; the host tabulates them per state with glibc.
-    const int rf = p.rfnum;
+    amt = jm * fdt2;
+    if (amt > p.ERODEFACTOR) amt = p.ERODEFACTOR;
+    // the two sums over the cells (:3547-3571), formed state by state, and
+    // the ledger (k_runoff_inputs adds amt to each computed cell of state z);
+    // new_jmeanmax (:3575-3586) over the states that hold a computed cell
+    const double got = cdiv(amt, fdt2);
+#pragma unroll 1
+    for (int z = 0; z <= rf; z++)
+      waterinput += c.runoff_count[z] * (__shfl_sync(FULL, jm, z) * DX * DX);
+#pragma unroll 1
     for (int z = 0; z <= rf; z++) {
-      double amt = s.j_mean[z] * fdt2;
-      if (amt > p.ERODEFACTOR) amt = p.ERODEFACTOR;
-      d->input_amt[z] = amt;
-      d->j_mean_in[z] = s.j_mean[z];
+      const double n = c.runoff_count[z];
+      waterinput += n * (__shfl_sync(FULL, got, z) * DX * DX);
+      const double a = __shfl_sync(FULL, amt, z), v = __shfl_sync(FULL, newj, z);
+      if (n > 0) vin += n * a;
+      if (((c.runoff_present >> z) & 1u) && v > jmm) jmm = v;
     }
-    // the two sums over the cells (:3547-3571), formed state by state
-    for (int z = 0; z <= rf; z++) s.waterinput += c.runoff_count[z] * (s.j_mean[z] * DX * DX);
-    for (int z = 0; z <= rf; z++)
-      s.waterinput += c.runoff_count[z] * ((d->input_amt[z] / fdt2) * DX * DX);
-    // ledger: k_runoff_inputs adds input_amt[z] to each computed cell of state z
-    for (int z = 0; z <= rf; z++)
-      if (c.runoff_count[z] > 0) d->vin_step += c.runoff_count[z] * d->input_amt[z];
-    d->input_dt = fdt2;
-    // new_jmeanmax (:3575-3586), over the states that hold a computed cell
-    double jmm = 0;
-    for (int z = 0; z <= rf; z++)
-      if (((c.runoff_present >> z) & 1u) && s.new_j_mean[z] > jmm) jmm = s.new_j_mean[z];
-    if (s.cycle >= s.time_1) {
-      do {
-        s.time_1++;
-        topmodel_step(d, p, c.topm, c.topm_rows);
-        if (s.time_step > p.max_time_step &&
-            jmm > (0.2 / ((unsigned)p.jmax * (unsigned)p.imax * DX * DX))) {
-          s.cycle = s.time_1 + (p.max_time_step / 60);
-          s.time_step = p.max_time_step;
-        }
-      } while (s.time_1 < s.cycle && !(d->pause & HC_PAUSE_ERROR));
-    }
-    for (int z = 0; z <= rf; z++)  // calchydrograph(time, runoff) :3728-3740
-      s.j_mean[z] = s.old_j_mean[z] + (((s.new_j_mean[z] - s.old_j_mean[z]) / 2) *
-                                       (2 - (s.time_1 - s.cycle)));
-    d->do_drain = 0;  // no drainage area or input points in this mode
   } else {
-    for (int i = 1; i <= p.rfnum; i++) s.waterinput += s.j_mean[i] * s.nActualGridCells[i] * DX * DX;
-    for (int i = 0; i <= p.rfnum; i++) d->j_mean_in[i] = s.j_mean[i];
-    if (arec)
-      for (int i = 0; i <= HC_MAX_RF; i++) arec[3 + i] = (i <= p.rfnum) ? s.j_mean[i] : 0.0;
-    d->input_dt = fdt2;
+    const double flow = jm * cells;
+#pragma unroll 1
+    for (int i = 1; i <= rf; i++) waterinput += __shfl_sync(FULL, flow, i) * DX * DX;
     // what each input point of a zone receives (:3463-3477), the same for all
     // points of the zone
-    for (int z = 0; z <= p.rfnum && z <= HC_MAX_RF; z++) {
-      double amt = (d->j_mean_in[z] * s.nActualGridCells[z]) / (s.catchment_input_counter[z]) * fdt2;
-      if (amt > p.ERODEFACTOR) amt = p.ERODEFACTOR;
-      d->input_amt[z] = amt;
-    }
-    if (s.cycle >= s.time_1) {
-      do {
-        s.time_1++;
-        topmodel_step(d, p, c.topm, c.topm_rows);
-        if (s.time_step > p.max_time_step) {
-          double jmm = 0;
-          for (int n = 1; n <= p.rfnum; n++)
-            if (s.new_j_mean[n] > jmm) jmm = s.new_j_mean[n];
-          if (jmm > (0.2 / ((unsigned)p.imax * (unsigned)p.jmax * DX * DX))) {
-            s.cycle = s.time_1 + (p.max_time_step / 60);
-            s.time_step = p.max_time_step;
+    amt = cdiv(flow, points) * fdt2;
+    if (amt > p.ERODEFACTOR) amt = p.ERODEFACTOR;
+    if (arec && lane <= HC_MAX_RF) arec[3 + lane] = zone ? jm : 0.0;
+  }
+  if (zone) d->input_amt[lane] = amt;
+  if (cycle >= time_1) {
+    do {
+      time_1++;
+      // topmodel_runoff(time_1) :3649-3715: the recurrence depends only on
+      // the rain table, so the host evaluates it once (host_topmodel_table)
+      // and the device steps through the rows
+      const int t = (int)time_1;
+      if (t < 0 || t >= c.topm_rows) {
+        err = 101;
+        pause |= HC_PAUSE_ERROR;
+      } else if (zone && lane >= z0) {
+        const double* row = c.topm + (size_t)t * 2 * (rf + 1);
+        oldj = row[lane];
+        newj = row[(rf + 1) + lane];
+      }
+      if (time_step > p.max_time_step) {
+        if (!grid) {
+          jmm = 0;
+#pragma unroll 1
+          for (int n = 1; n <= rf; n++) {
+            const double v = __shfl_sync(FULL, newj, n);
+            if (v > jmm) jmm = v;
           }
         }
-      } while (s.time_1 < s.cycle && !(d->pause & HC_PAUSE_ERROR));
-    }
-    for (int n = 1; n <= p.rfnum; n++)  // calchydrograph :3718
-      s.j_mean[n] = s.old_j_mean[n] + (((s.new_j_mean[n] - s.old_j_mean[n]) / 2) * (2 - (s.time_1 - s.cycle)));
-    if (arec) {
-      arec[HC_ADJ_T1] = s.time_1;
-      arec[HC_ADJ_T1 + 1] = s.cycle;
+        if (jmm > cdiv(0.2, (unsigned)p.imax * (unsigned)p.jmax * DX * DX)) {
+          cycle = time_1 + (p.max_time_step / 60);
+          time_step = p.max_time_step;
+        }
+      }
+    } while (time_1 < cycle && !(pause & HC_PAUSE_ERROR));
+  }
+  // calchydrograph :3718 and (time, runoff) :3728-3740 (x / 2 == x * 0.5)
+  if (zone && lane >= z0) jm = oldj + (((newj - oldj) * 0.5) * (2 - (time_1 - cycle)));
+  bool recalc = false;  // no drainage area or input points with grid runoff
+  if (!grid) {
+    if (arec && l0) {
+      arec[HC_ADJ_T1] = time_1;
+      arec[HC_ADJ_T1 + 1] = cycle;
     }
     double jmeanmax = 0;
-    for (int n = 1; n <= p.rfnum; n++)
-      if (s.j_mean[n] > jmeanmax) jmeanmax = s.j_mean[n];
-    bool recalc = false;
-    if (jmeanmax >= s.baseflow) {
-      s.baseflow = s.baseflow * 3;
+#pragma unroll 1
+    for (int n = 1; n <= rf; n++) {
+      const double v = __shfl_sync(FULL, jm, n);
+      if (v > jmeanmax) jmeanmax = v;
+    }
+    if (jmeanmax >= baseflow) {
+      baseflow = baseflow * 3;
       recalc = true;
     }
-    if (s.baseflow > (jmeanmax * 3) && s.baseflow > 0.000001) {
-      s.baseflow = jmeanmax * 1.25;
+    if (baseflow > (jmeanmax * 3) && baseflow > 0.000001) {
+      baseflow = jmeanmax * 1.25;
       recalc = true;
     }
     // The drainage area and the input-point list are recomputed before the
@@ -244,37 +279,64 @@ __global__ void k_control(const hc_view c, hc_dev* d, hc_iter_handles hh) {
     // rest), from the elevations as they are now (k_depth_update copies
     // them before the iteration's erosion); the
     // reference, too, applies the new list from the next iteration on.
-    d->do_drain = recalc;
-    if (recalc) d->pause |= HC_PAUSE_DRAINAGE;
+    if (recalc) pause |= HC_PAUSE_DRAINAGE;
+  }
+  if (zone && lane >= z0) {
+    s.j_mean[lane] = jm;
+    s.old_j_mean[lane] = oldj;
+    s.new_j_mean[lane] = newj;
   }
 
-  s.flow_timestep = flow_dt_of(p, s);
+  double flow_timestep = time_step > cfl ? cfl : time_step;
+  if (impose) flow_timestep = arec[2];
+  const bool scan = divides(counter, p.scan_area_interval_iter);
+  const bool erode = !p.hydro_only && counter >= erode_call;
+  const bool slide = !p.hydro_only && divides(counter, p.in_channel_landslide_iter_interval);
+  if (!l0) return;
   if (adj) {
-    if (d->adj_mode == 2) s.flow_timestep = arec[2];
-    else arec[2] = s.flow_timestep;
+    if (!impose) arec[2] = flow_timestep;
     d->adj_i++;
   }
-  d->do_scan = ((long long)s.counter % p.scan_area_interval_iter) == 0;
-  d->do_erode = !p.hydro_only && s.counter >= s.erode_call;
-  d->erode_retry = d->do_erode;
-  if (d->do_erode) {
+  d->budget = budget - 1;
+  d->it_active = 1;
+  d->rest_active = 1;
+  d->erode_passes = 0;
+  d->do_lateral = 0;
+  d->do_drain = recalc;
+  d->do_scan = scan;
+  d->do_erode = erode;
+  d->erode_retry = erode;
+  d->do_slide = slide;
+  if (pause) d->pause = pause;
+  if (err) d->err_code = err;
+  d->input_dt = fdt2;
+  d->vin_step = vin;
+  s.previous = previous;
+  s.input_output_difference = diff;
+  s.maxdepth = maxdepth;
+  s.counter = counter;
+  s.cycle = cycle;
+  s.time_1 = time_1;
+  s.waterinput = waterinput;
+  s.baseflow = baseflow;
+  s.flow_timestep = flow_timestep;
+  if (erode) {
     // erode()'s start (:4219; k_erode_begin for a direct call): the
     // kernels between here and the erosion block read flow_timestep, set
     // above, not time_step
-    s.time_step = s.time_step * 1.5;
-    d->mult = s.erode_mult;
+    time_step = time_step * 1.5;
+    d->mult = erode_mult;
     d->tempbmax_bits = 0;
   }
-  d->do_slide = !p.hydro_only && ((long long)s.counter % p.in_channel_landslide_iter_interval) == 0;
+  s.time_step = time_step;
   if (hh.has) {
     // kernels inside the bodies enabled here: scan 3, erosion 5 + 7, slide_3 4
-    d->body_kernels += (d->do_scan ? 3 : 0) + (d->do_erode && !p.hydro_only ? 12 : 0) +
-                       (d->do_slide ? 4 : 0);
-    cudaGraphSetConditional(hh.scan, d->do_scan ? 1u : 0u);
+    d->body_kernels += (scan ? 3 : 0) + (erode ? 12 : 0) + (slide ? 4 : 0);
+    cudaGraphSetConditional(hh.scan, scan ? 1u : 0u);
     if (!p.hydro_only) {
-      cudaGraphSetConditional(hh.erode, d->do_erode ? 1u : 0u);
-      cudaGraphSetConditional(hh.erode_fin, d->do_erode ? 1u : 0u);
-      cudaGraphSetConditional(hh.slide, d->do_slide ? 1u : 0u);
+      cudaGraphSetConditional(hh.erode, erode ? 1u : 0u);
+      cudaGraphSetConditional(hh.erode_fin, erode ? 1u : 0u);
+      cudaGraphSetConditional(hh.slide, slide ? 1u : 0u);
     }
   }
 }
@@ -1131,7 +1193,7 @@ static dim3 grid2d(const hc_ctx* c, dim3 b) {
 }
 
 void launch_control(hc_ctx* c) {
-  k_control<<<1, 1, 0, c->cs>>>(c->v, c->dev, c->hcur);
+  k_control<<<1, 32, 0, c->cs>>>(c->v, c->dev, c->hcur);
   count_launch(c, 1);
 }
 
