@@ -77,7 +77,6 @@ struct hc_dev {
   int flags;              // HC_RUN_* of the current run
   unsigned int depth_done;   // blocks finished in depth_update (last-block reduction)
   unsigned int pass_done;    // blocks finished in an entrainment pass
-  unsigned int misc_done;
   // arrival counters of the launches whose last block finishes the step
   // (last_to_arrive): the wet list's count, the grain records' count and
   // assignment, slide_3's flag count, the edge outflow; each is zero between launches
