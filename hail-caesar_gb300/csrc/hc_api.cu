@@ -74,6 +74,11 @@ __global__ void k_fill_d(double* a, size_t n, double v) {
        i += (size_t)gridDim.x * blockDim.x)
     a[i] = v;
 }
+__global__ void k_square(const double* a, double* b, size_t n) {
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+       i += (size_t)gridDim.x * blockDim.x)
+    b[i] = a[i] * a[i];
+}
 __global__ void k_fill_i(int32_t* a, size_t n, int32_t v) {
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (size_t)gridDim.x * blockDim.x)
@@ -241,6 +246,8 @@ extern "C" hc_status hc_create(const hc_params* p, size_t max_bytes, hc_ctx** ou
   v.p = *p;
   v.rDX = 1.0 / p->DX;
   v.dxd = host_divisor(p->DX);
+  v.fived = host_divisor(5.0);
+  v.nn = p->mannings * p->mannings;
   v.DXf = (float)p->DX;
   v.flf = (float)p->froude_limit;
   v.act_hi = (float)(p->active * 1.5);
@@ -280,7 +287,7 @@ extern "C" hc_status hc_create(const hc_params* p, size_t max_bytes, hc_ctx** ou
 #define A(ptr, n)                                    \
   if (st == HC_OK) st = dalloc(c, &(ptr), (n));
   A(v.elev, N2) A(v.h, N2) A(v.qx, N2) A(v.qy, N2) A(v.qxs, N2) A(v.qys, N2) A(v.vs, N2)
-  A(v.vel, N2) A(v.tau, N2) A(v.bed, N2) A(v.man, N2) A(v.area, N2) A(v.ss, N2)
+  A(v.vel, N2) A(v.tau, N2) A(v.bed, N2) A(v.man, N2) A(v.man2, N2) A(v.area, N2) A(v.ss, N2)
   A(v.vd, 4 * N2) A(v.index, N2) A(v.mask, N2) A(v.border, N2) A(v.rfarea, N2)
   A(v.edge, E2) A(v.edge2, E2) A(v.veg, 4 * E2)
   A(v.cin_x, (size_t)p->imax * p->jmax + 2) A(v.cin_y, (size_t)p->imax * p->jmax + 2)
@@ -321,7 +328,7 @@ extern "C" hc_status hc_create(const hc_params* p, size_t max_bytes, hc_ctx** ou
   }
   // zero_values :2891-2982
   cudaStream_t s = c->s;
-  for (double* a : {v.h, v.qx, v.qy, v.qxs, v.qys, v.vs, v.vel, v.tau, v.man, v.area, v.ss})
+  for (double* a : {v.h, v.qx, v.qy, v.qxs, v.qys, v.vs, v.vel, v.tau, v.man, v.man2, v.area, v.ss})
     cudaMemsetAsync(a, 0, N2 * 8, s);
   fill_d(c, v.elev, N2, -9999);
   fill_d(c, v.bed, N2, -9999);
@@ -375,7 +382,7 @@ extern "C" hc_status hc_create(const hc_params* p, size_t max_bytes, hc_ctx** ou
 
 static hc_status free_all(hc_ctx* c) {
   hc_view& v = c->v;
-  void* ptrs[] = {v.elev, v.h, v.qx, v.qy, v.qxs, v.qys, v.vs, v.vel, v.tau, v.bed, v.man,
+  void* ptrs[] = {v.elev, v.h, v.qx, v.qy, v.qxs, v.qys, v.vs, v.vel, v.tau, v.bed, v.man, v.man2,
                   v.area, v.ss, v.vd, v.sflux, v.grain, v.strata, v.index, v.mask, v.rfarea,
                   v.edge, v.edge2, v.veg, v.cin_x, v.cin_y, v.erodetot, v.erodetot3, v.pre,
                   v.chains, v.ent_list, v.ent_qs, v.drain_pos, v.drain_f0, v.drain_f1, v.drain_pend, v.drain_dt, v.drain_share, v.drain_head,
@@ -461,6 +468,8 @@ extern "C" hc_status hc_upload(hc_ctx* c, hc_field f, const void* host, size_t n
   cudaStream_t s = c->s;
   if (double* d = plain_field(c, f)) {
     HC_CU(cudaMemcpyAsync(d, host, nbytes, cudaMemcpyHostToDevice, s), "upload");
+    if (f == HC_F_MANNINGS)
+      k_square<<<(unsigned)std::min<size_t>((N2 + 255) / 256, 4096), 256, 0, s>>>(v.man, v.man2, N2);
     HC_CU(cudaStreamSynchronize(s), "upload");
     if (f == HC_F_ELEV || f == HC_F_AREA) c->area_valid = false;
     if (f == HC_F_ELEV && c->drainage_cache) {  // the cached elevation order is stale

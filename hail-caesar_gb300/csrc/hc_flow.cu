@@ -395,33 +395,29 @@ struct FaceOut {
 // decide them: out of line, so that their FP64 instructions (a hardware
 // division among them) issue only where they run.
 static __device__ __noinline__ bool depth_exceeds(double qn, double dt, double DX, double h) {
-  return (qn * dt / DX) > (h / 4);  // :3138, :3218
-}
-static __device__ __noinline__ bool depth_exceeds_neg(double qn, double dt, double DX, double h) {
-  return fabs(qn * dt / DX) > (h / 4);  // :3144, :3219
+  return fabs(qn * dt / DX) > (h / 4);  // :3138, :3144, :3218, :3219
 }
 static __device__ __noinline__ bool sed_exceeds(double qs, double dt, double v, double DX) {
-  return qs * dt > (v * DX) / 4;  // :3163
-}
-static __device__ __noinline__ bool sed_exceeds_neg(double qs, double dt, double v, double DX) {
-  return fabs(qs * dt) > (v * DX) / 4;  // :3169
+  return fabs(qs * dt) > (v * DX) / 4;  // :3163, :3169
 }
 
 // The limiters' replacement values and the Froude test's exact form, out of
 // line as well: they run for few faces, and inlined, their integer-pipe
 // divisions and square roots would double the kernel's code, whose
 // instruction fetches stall the warps more than anything else.
-// (x * DX / 5) / dt, the depth and sediment limits' value (:3140, :3165)
-static __device__ __noinline__ double limit_value(double x, double DX, double dt) {
-  return ddiv_rn(ddiv_rn(x * DX, 5.0), dt);
+// (x * DX / 5) / dt, the depth and sediment limits' value (:3140, :3165);
+// the divisors 5 (host) and dt (once per block) come prepared
+static __device__ __noinline__ double limit_value(double x, const hc_view& c,
+                                                  const hc_divisor* dtd) {
+  return ddiv_by(ddiv_by(x * c.p.DX, c.fived), *dtd);
 }
-// |q/hflow| / sqrt(g hflow) > froude_limit, exactly (:3124)
-static __device__ __noinline__ bool froude_exceeds(double qoh, double hflow, double fl) {
-  return dgt(ddiv_rn(fabs(qoh), isqrt_rn(kG * hflow)), fl);
+// |q/hflow| / sqrt(g hflow) > froude_limit, exactly (:3124); gh = g hflow
+static __device__ __noinline__ bool froude_exceeds(double qoh, double gh, double fl) {
+  return dgt(ddiv_rn(fabs(qoh), isqrt_rn(gh)), fl);
 }
 // hflow * (sqrt(g hflow) * froude_limit), the Froude limit's value (:3127)
-static __device__ __noinline__ double froude_value(double hflow, double fl) {
-  return hflow * (isqrt_rn(kG * hflow) * fl);
+static __device__ __noinline__ double froude_value(double hflow, double gh, double fl) {
+  return hflow * (isqrt_rn(gh) * fl);
 }
 
 // Three-way test of A > B from float estimates a, b, each within a relative
@@ -468,14 +464,15 @@ __device__ __forceinline__ void inertial_face_core(double& q, double& qs, double
                                                    int& vdir, double hflow, double dA, double h0,
                                                    double h1, double v0, double v1, double c0,
                                                    double nn, double dt, int edge_slope,
-                                                   const hc_view& c) {
+                                                   const hc_view& c, const hc_divisor* dtd) {
   const hc_params& p = c.p;
   const double DX = p.DX;
   vdir = 0;
   double slope = ddiv_by(dA, c.dxd);
   if (edge_slope == 1) slope = p.edgeslope;
   if (edge_slope == -1) slope = zero_minus(p.edgeslope);
-  const double ghd = kG * hflow * dt;
+  const double gh = kG * hflow;
+  const double ghd = gh * dt;
   // the numerator once for both branches (a branch apiece would issue its
   // FP64 instructions twice in a warp that holds both)
   double qn = q - (ghd * slope);
@@ -503,47 +500,52 @@ __device__ __forceinline__ void inertial_face_core(double& q, double& qs, double
     int t = decide_gt(fr, c.flf);
     if (t == 0) {
       if (!qoh_valid) qoh = fdiv<kCall>(qn, hflow);
-      t = froude_exceeds(qoh, hflow, p.froude_limit) ? 1 : -1;
+      t = froude_exceeds(qoh, gh, p.froude_limit) ? 1 : -1;
     }
     if (t > 0) {
-      const double lim = froude_value(hflow, p.froude_limit);
+      const double lim = froude_value(hflow, gh, p.froude_limit);
       qn = dgt0(qn) ? lim : zero_minus(lim);
       qoh_valid = false;
     }
   }
-  // depth limit: |q*dt/DX| > (depth of the giving cell)/4; the two tests
-  // run one after the other, as in the reference
-  if (dgt0(qn)) {
-    int t = decide_gt(approx_abs_f(qn) * dtf / c.DXf, approx_f(h0) * 0.25f);
-    if (t == 0) t = depth_exceeds(qn, dt, DX, h0) ? 1 : -1;
+  // depth limit: |q*dt/DX| > (depth of the giving cell)/4.  The reference
+  // tests q > 0, then q < 0 on what that left; a limited q keeps its sign
+  // when its depth is not negative, so one test of the giving cell serves
+  // both, and a warp issues the limit's operations once.  Only a negative
+  // depth lets the first test's result reach the second.
+  auto depth_limit = [&](double h, bool pos) {
+    int t = decide_gt(approx_abs_f(qn) * dtf / c.DXf, approx_f(h) * 0.25f);
+    if (t == 0) t = depth_exceeds(qn, dt, DX, h) ? 1 : -1;
     if (t > 0) {
-      qn = limit_value(h0, DX, dt);
+      const double lim = limit_value(h, c, dtd);
+      qn = pos ? lim : zero_minus(lim);
       qoh_valid = false;
     }
-  }
-  if (dlt0(qn)) {
-    int t = decide_gt(approx_abs_f(qn) * dtf / c.DXf, approx_f(h1) * 0.25f);
-    if (t == 0) t = depth_exceeds_neg(qn, dt, DX, h1) ? 1 : -1;
-    if (t > 0) {
-      qn = zero_minus(limit_value(h1, DX, dt));
-      qoh_valid = false;
-    }
+  };
+  if (!deq0(qn)) {
+    const bool pos = dgt0(qn);
+    depth_limit(pos ? h0 : h1, pos);
+    if (pos && dlt0(qn)) depth_limit(h1, false);
   }
   const bool qpos = dgt0(qn), qneg = dlt0(qn);
   if (kSusp) {
     // qs = q * (V/h) of the giving cell; V = 0 gives 0 * q (a signed zero)
     // (one product for both signs: h1 > 0 here, as h0 above)
     if (qpos || qneg) qs = qn * (qpos ? c0 : (deq0(v1) ? v1 : fdiv<kCall>(v1, h1)));
-    // qs*dt > V*DX/4 (giving cell) caps the sediment flux
-    if (dgt0(qs)) {
-      int t = decide_gt(approx_abs_f(qs) * dtf, approx_f(v0) * c.DXf * 0.25f);
-      if (t == 0) t = sed_exceeds(qs, dt, v0, DX) ? 1 : -1;
-      if (t > 0) qs = limit_value(v0, DX, dt);
-    }
-    if (dlt0(qs)) {
-      int t = decide_gt(approx_abs_f(qs) * dtf, approx_f(v1) * c.DXf * 0.25f);
-      if (t == 0) t = sed_exceeds_neg(qs, dt, v1, DX) ? 1 : -1;
-      if (t > 0) qs = zero_minus(limit_value(v1, DX, dt));
+    // qs*dt > V*DX/4 (giving cell) caps the sediment flux, the two signs'
+    // tests as one like the depth limit's
+    auto sed_limit = [&](double v, bool pos) {
+      int t = decide_gt(approx_abs_f(qs) * dtf, approx_f(v) * c.DXf * 0.25f);
+      if (t == 0) t = sed_exceeds(qs, dt, v, DX) ? 1 : -1;
+      if (t > 0) {
+        const double lim = limit_value(v, c, dtd);
+        qs = pos ? lim : zero_minus(lim);
+      }
+    };
+    if (!deq0(qs)) {
+      const bool pos = dgt0(qs);
+      sed_limit(pos ? v0 : v1, pos);
+      if (pos && dlt0(qs)) sed_limit(v1, false);
     }
   }
   if (kVel) {
@@ -566,7 +568,7 @@ __device__ __forceinline__ void inertial_face(double& q, double& qs, double& vel
                                               double e0, double h0, double a0, double e1,
                                               double h1, double a1, double v0, double v1,
                                               double c0, double nn, double dt, int edge_slope,
-                                              const hc_view& c) {
+                                              const hc_view& c, const hc_divisor* dtd) {
   vdir = 0;
   double hflow = imax_d(a0, a1) - imax_d(e1, e0);
   if (!(dkey(hflow) > c.thr_key)) {  // hflow > hflow_threshold
@@ -575,12 +577,12 @@ __device__ __forceinline__ void inertial_face(double& q, double& qs, double& vel
     return;
   }
   inertial_face_core<kSusp, kVel>(q, qs, vel_out, vdir, hflow, a1 - a0, h0, h1, v0, v1, c0, nn,
-                                  dt, edge_slope, c);
+                                  dt, edge_slope, c, dtd);
 }
 
 template <bool kSed>
 __device__ __forceinline__ void flow_cell(const hc_view& c, const hc_dev* __restrict__ d,
-                                          size_t cell) {
+                                          size_t cell, const hc_divisor* dtd) {
   const size_t W = c.W, N2 = c.N2;
   const int i = (int)(cell / W), j = (int)(cell % W);
   const double e0 = c.elev[cell];
@@ -589,8 +591,7 @@ __device__ __forceinline__ void flow_cell(const hc_view& c, const hc_dev* __rest
   if (!above_nodata(e0)) return;
   const hc_params& p = c.p;
   const double dt = d->s.flow_timestep;
-  const double n = p.spatially_var_mannings ? c.man[cell] : p.mannings;
-  const double nn = n * n;
+  const double nn = p.spatially_var_mannings ? c.man2[cell] : c.nn;  // n * n
   const bool susp = kSed && p.isSuspended[1] != 0;
   const double h0 = c.h[cell];
   const double a0 = e0 + h0;
@@ -610,10 +611,10 @@ __device__ __forceinline__ void flow_cell(const hc_view& c, const hc_dev* __rest
       const int es = (i == c.imax) ? 1 : ((i <= 2) ? -1 : 0);
       if (susp)
         inertial_face<true, kSed>(q, qs, vel, vdir, e0, h0, a0, e1, h1, e1 + h1, v0, c.vs[up],
-                                  c0, nn, dt, es, c);
+                                  c0, nn, dt, es, c, dtd);
       else
         inertial_face<false, kSed>(q, qs, vel, vdir, e0, h0, a0, e1, h1, e1 + h1, v0, 0.0, c0,
-                                   nn, dt, es, c);
+                                   nn, dt, es, c, dtd);
       c.qx[cell] = q;
       if (kSed) {
         c.qxs[cell] = qs;
@@ -634,10 +635,10 @@ __device__ __forceinline__ void flow_cell(const hc_view& c, const hc_dev* __rest
       const int es = (j == c.jmax) ? 1 : ((j <= 2) ? -1 : 0);
       if (susp)
         inertial_face<true, kSed>(q, qs, vel, vdir, e0, h0, a0, e1, h1, e1 + h1, v0, c.vs[lf],
-                                  c0, nn, dt, es, c);
+                                  c0, nn, dt, es, c, dtd);
       else
         inertial_face<false, kSed>(q, qs, vel, vdir, e0, h0, a0, e1, h1, e1 + h1, v0, 0.0, c0,
-                                   nn, dt, es, c);
+                                   nn, dt, es, c, dtd);
       c.qy[cell] = q;
       if (kSed) {
         c.qys[cell] = qs;
@@ -656,9 +657,12 @@ template <bool kSed, int MINB>
 __global__ void __launch_bounds__(256, MINB) k_flow_route(const hc_view c,
                                                           const hc_dev* __restrict__ d, int gated) {
   if (gated && !d->it_active) return;
+  __shared__ hc_divisor dtd;  // dt as a divisor, for the limits
+  if (threadIdx.x == 0) dtd = ddiv_prep(d->s.flow_timestep);
+  __syncthreads();
   const int n = d->wet_count;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x)
-    flow_cell<kSed>(c, d, (size_t)c.wet[k]);
+    flow_cell<kSed>(c, d, (size_t)c.wet[k], &dtd);
 }
 
 // Face-compacted flow_route.  In a storm about half the listed cells are dry
@@ -675,7 +679,7 @@ __global__ void __launch_bounds__(256, MINB) k_flow_route(const hc_view c,
 constexpr int kFaceQ = 96;  // queue entries per warp: < 32 carried + 64 new
 
 template <bool kSed, bool kCall>
-__device__ __forceinline__ void face_work(const hc_view& c, const hc_dev* __restrict__ d,
+__device__ __forceinline__ void face_work(const hc_view& c, const hc_divisor* dtd,
                                           uint32_t f, double hflow, double dA, double dt) {
   const size_t W = c.W, N2 = c.N2;
   const size_t cell = f >> 1;
@@ -683,8 +687,7 @@ __device__ __forceinline__ void face_work(const hc_view& c, const hc_dev* __rest
   const size_t nb = yface ? cell - 1 : cell - W;
   const int i = (int)(cell / W), j = (int)(cell - (size_t)i * W);
   const hc_params& p = c.p;
-  const double n = p.spatially_var_mannings ? c.man[cell] : p.mannings;
-  const double nn = n * n;
+  const double nn = p.spatially_var_mannings ? c.man2[cell] : c.nn;  // n * n
   const bool susp = kSed && p.isSuspended[1] != 0;
   const double h0 = c.h[cell], h1 = c.h[nb];
   const double v0 = susp ? c.vs[cell] : 0.0;
@@ -697,10 +700,10 @@ __device__ __forceinline__ void face_work(const hc_view& c, const hc_dev* __rest
                        : ((i == c.imax) ? 1 : ((i <= 2) ? -1 : 0));
   if (susp)
     inertial_face_core<true, kSed, kCall>(q, qs, vel, vdir, hflow, dA, h0, h1, v0, c.vs[nb], c0, nn,
-                                   dt, es, c);
+                                          dt, es, c, dtd);
   else
     inertial_face_core<false, kSed, kCall>(q, qs, vel, vdir, hflow, dA, h0, h1, v0, 0.0, c0, nn, dt,
-                                    es, c);
+                                           es, c, dtd);
   qa[cell] = q;
   if (kSed) {
     qsa[cell] = qs;
@@ -716,7 +719,10 @@ __global__ void __launch_bounds__(256, MINB) k_flow_route_q(const hc_view c,
                                                             int gated) {
   __shared__ uint32_t qf[8][kFaceQ];
   __shared__ double qh[8][kFaceQ], qa[8][kFaceQ];
+  __shared__ hc_divisor dtd;  // dt as a divisor, for the limits
   if (gated && !d->it_active) return;
+  if (threadIdx.x == 0) dtd = ddiv_prep(d->s.flow_timestep);
+  __syncthreads();
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint32_t* Q = qf[warp];
@@ -797,10 +803,10 @@ __global__ void __launch_bounds__(256, MINB) k_flow_route_q(const hc_view c,
       const uint32_t f = Q[qn + lane];
       const double hf = HF[qn + lane], da = DA[qn + lane];
       __syncwarp();  // the entries are read before the next cells' are written
-      face_work<kSed, kCall>(c, d, f, hf, da, dt);
+      face_work<kSed, kCall>(c, &dtd, f, hf, da, dt);
     }
   }
-  if (lane < qn) face_work<kSed, kCall>(c, d, Q[lane], HF[lane], DA[lane], dt);
+  if (lane < qn) face_work<kSed, kCall>(c, &dtd, Q[lane], HF[lane], DA[lane], dt);
 }
 
 // ---------------------------------------------------------------------------

@@ -132,7 +132,8 @@ struct hc_divisor {
 struct hc_view {
   hc_params p;
   double rDX;             // RN(1/DX) (the adjoint's slope derivatives)
-  hc_divisor dxd;         // DX as a divisor (ddiv_by)
+  hc_divisor dxd, fived;  // DX and 5 as divisors (ddiv_by)
+  double nn;              // mannings * mannings (one n for all cells)
   float DXf, flf;         // DX and froude_limit as floats (estimates only)
   float act_hi, act_lo;   // (float)(active*1.5), (float)(active/4): sort_active's estimates
   long long thr_key;      // dkey(hflow_threshold)
@@ -141,6 +142,7 @@ struct hc_view {
 
   // fields
   double *elev, *h, *qx, *qy, *qxs, *qys, *vs, *vel, *tau, *bed, *man, *area, *ss;
+  double *man2;      // man * man, kept beside it for flow_route
   double *vd;        // 4 * N2
   double *sflux;     // 4 dirs * 10 fractions * N2 ; dir order su, sr, sd, sl
   uint8_t *sdirty;   // N2: 1 where the cell's sflux entries may be nonzero
