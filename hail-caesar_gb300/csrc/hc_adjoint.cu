@@ -118,7 +118,7 @@ __device__ DQ face_dq(double q, double hflow, double dA, bool e0max, H0 h0f, H1 
     d_s = -ghd;
     d_nn = 0;
   } else {
-    const double aq = __longlong_as_double(dbits(q) & 0x7fffffffffffffffLL);  // fabs
+    const double aq = bits_d(dbits(q) & 0x7fffffffffffffffLL);  // fabs
     const double c3 = icube_rn(hflow);
     const double F = adj_div(ghd * nn * aq, c3);
     const double D = 1 + F, N = q - (ghd * slope);

@@ -49,7 +49,7 @@ __host__ __device__ __forceinline__ unsigned long long ukey_bits(long long b) {
   return (unsigned long long)k ^ 0x8000000000000000ULL;
 }
 __device__ __forceinline__ unsigned long long ukey(double x) {
-  return ukey_bits(__double_as_longlong(x));
+  return ukey_bits(dbits(x));
 }
 constexpr unsigned long long kZeroKey = 0x8000000000000000ULL;  // ukey(0.0)
 
@@ -267,7 +267,7 @@ __global__ void k_drain_terms(const hc_view c, const double* __restrict__ el) {
   }
   c.drain_head[cell] = head | ((unsigned long long)n << kHeadCount);
   // not yet summed: no area is a NaN
-  c.area[cell] = __longlong_as_double(-1LL);
+  c.area[cell] = bits_d(-1LL);
 }
 
 // The sweep's shared state, all zero at the start but `tail`.
@@ -408,7 +408,7 @@ __global__ void __launch_bounds__(kSweepThreads) k_drain_sweep(const hc_view c, 
 #pragma unroll
       for (int t = 0; t < 8; t++)  // the terms past n are +0, which adds nothing
         if (t < n_warp)
-          sum += __longlong_as_double((long long)a[t]) * __longlong_as_double((long long)s[t]);
+          sum += bits_d((long long)a[t]) * bits_d((long long)s[t]);
       if (!((head >> kHeadReached) & 1u) || !(sum > 0)) sum = 0;
       st_relaxed(c.area + cell, (unsigned long long)dbits(sum));
       // second round trip: the lower neighbours' counts and heads

@@ -324,7 +324,7 @@ __global__ void __launch_bounds__(128) k_entrain(const hc_view c, hc_dev* d, int
   __syncthreads();
   if (last && t == 0) {
     __threadfence();
-    const double tempbmax = __longlong_as_double((long long)atomicExch(&d->tempbmax_bits, 0ull));
+    const double tempbmax = bits_d((long long)atomicExch(&d->tempbmax_bits, 0ull));
     d->pass_done = 0;
     d->ent_n = 0;
     d->erode_passes++;

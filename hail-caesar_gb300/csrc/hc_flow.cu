@@ -478,7 +478,7 @@ __device__ __forceinline__ void inertial_face_core(double& q, double& qs, double
   double qn = q - (ghd * slope);
   // q = 0: (0 - ghd*slope) / (1 + (ghd*nn*0)/h^3) = (0 - ghd*slope) / 1
   if (!deq0(q)) {
-    const double aq = __longlong_as_double(dbits(q) & 0x7fffffffffffffffLL);  // fabs
+    const double aq = bits_d(dbits(q) & 0x7fffffffffffffffLL);  // fabs
     qn = fdiv<kCall>(qn, 1 + fdiv<kCall>(ghd * nn * aq, icube_rn(hflow)));
   }
   const float hf = approx_abs_f(hflow);
@@ -914,7 +914,7 @@ __global__ void __launch_bounds__(256, 6) k_depth_update(const hc_view c, hc_dev
     const double etot = block_sum(a);
     if (t == 0) {
       unsigned long long bits = atomicExch(&d->maxdepth_bits, 0ull);
-      d->s.maxdepth = __longlong_as_double((long long)bits);
+      d->s.maxdepth = bits_d((long long)bits);
       d->maxdepth_step = d->s.maxdepth;
       d->vmask_step += etot;
       d->depth_done = 0;
@@ -1150,7 +1150,7 @@ __global__ void __launch_bounds__(kFluxThreads) k_flux_out(const hc_view c, hc_d
       r.vol_in = vin * a2;
       r.vol_out = (vpart[0] + vlost) * a2;
       r.vol_mask = vmask * a2;
-      r.volume = (vol_counter == r.counter) ? vol * a2 : __longlong_as_double(0x7ff8000000000000LL);
+      r.volume = (vol_counter == r.counter) ? vol * a2 : bits_d(0x7ff8000000000000LL);
       rec[d->rec_index] = r;
     }
     if (record) d->rec_index++;
