@@ -225,7 +225,8 @@ hc_divisor host_divisor(double b) {
   d.eb = (int)(B >> 52) & 0x7ff;
   d.ok = d.eb != 0 && d.eb != 0x7ff;
   d.mb = (B & (H52 - 1)) | H52;
-  d.V = (d.mb == H52) ? 0 : (unsigned long long)(((unsigned __int128)1 << 116) / d.mb);
+  // floor(2^116/mb); for a power of two, 2^64 - 1 (one unit less, as ddiv_by allows)
+  d.V = (d.mb == H52) ? ~0ull : (unsigned long long)(((unsigned __int128)1 << 116) / d.mb);
   return d;
 }
 
