@@ -258,6 +258,7 @@ extern "C" hc_status hc_create(const hc_params* p, size_t max_bytes, hc_ctx** ou
     std::memcpy(&b, &p->hflow_threshold, 8);
     const long long sgn = b >> 63;
     v.thr_key = ((b & 0x7fffffffffffffffLL) ^ sgn) - sgn;  // dkey on the host
+    v.thr_xkey = v.thr_key < 0 ? v.thr_key - 1 : v.thr_key;
   }
   for (int n = 1; n <= 9; n++) {
     const double Di = p->d[n], g = 9.81;

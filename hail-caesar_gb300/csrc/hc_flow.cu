@@ -570,8 +570,8 @@ __device__ __forceinline__ void inertial_face(double& q, double& qs, double& vel
                                               double c0, double nn, double dt, int edge_slope,
                                               const hc_view& c, const hc_divisor* dtd) {
   vdir = 0;
-  double hflow = imax_d(a0, a1) - imax_d(e1, e0);
-  if (!(dkey(hflow) > c.thr_key)) {  // hflow > hflow_threshold
+  double hflow = xmax_d(a0, a1) - xmax_d(e1, e0);
+  if (!(xkey(hflow) > c.thr_xkey)) {  // hflow > hflow_threshold
     q = 0;
     qs = 0;
     return;
@@ -587,7 +587,7 @@ __device__ __forceinline__ void flow_cell(const hc_view& c, const hc_dev* __rest
   const int i = (int)(cell / W), j = (int)(cell % W);
   const double e0 = c.elev[cell];
   // e > -9999 (no-data and below are skipped)
-  auto above_nodata = [](double e) { return dkey(e) > kNoDataKey; };
+  auto above_nodata = [](double e) { return xkey(e) > kNoDataXKey; };
   if (!above_nodata(e0)) return;
   const hc_params& p = c.p;
   const double dt = d->s.flow_timestep;
@@ -747,18 +747,18 @@ __global__ void __launch_bounds__(256, MINB) k_flow_route_q(const hc_view c,
     if (k < n) {
       cell = mine;
       const double e0 = c.elev[cell];
-      if (dkey(e0) > kNoDataKey) {  // e > -9999
+      if (xkey(e0) > kNoDataXKey) {  // e > -9999
         const double h0 = c.h[cell];
         const double a0 = e0 + h0;
         const bool wet0 = dgt0(h0);
         {
           const size_t up = cell - W;
           const double h1 = c.h[up], e1 = c.elev[up];
-          if ((wet0 || dgt0(h1)) && dkey(e1) > kNoDataKey) {
+          if ((wet0 || dgt0(h1)) && xkey(e1) > kNoDataXKey) {
             const double a1 = e1 + h1;
-            hx = imax_d(a0, a1) - imax_d(e1, e0);
+            hx = xmax_d(a0, a1) - xmax_d(e1, e0);
             ax = a1 - a0;
-            fx = dkey(hx) > c.thr_key;
+            fx = xkey(hx) > c.thr_xkey;
             if (!fx) {
               c.qx[cell] = 0;
               if (kSed) c.qxs[cell] = 0;
@@ -768,11 +768,11 @@ __global__ void __launch_bounds__(256, MINB) k_flow_route_q(const hc_view c,
         {
           const size_t lf = cell - 1;
           const double h1 = c.h[lf], e1 = c.elev[lf];
-          if ((wet0 || dgt0(h1)) && dkey(e1) > kNoDataKey) {
+          if ((wet0 || dgt0(h1)) && xkey(e1) > kNoDataXKey) {
             const double a1 = e1 + h1;
-            hy = imax_d(a0, a1) - imax_d(e1, e0);
+            hy = xmax_d(a0, a1) - xmax_d(e1, e0);
             ay = a1 - a0;
-            fy = dkey(hy) > c.thr_key;
+            fy = xkey(hy) > c.thr_xkey;
             if (!fy) {
               c.qy[cell] = 0;
               if (kSed) c.qys[cell] = 0;

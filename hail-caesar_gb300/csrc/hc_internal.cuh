@@ -136,7 +136,7 @@ struct hc_view {
   double nn;              // mannings * mannings (one n for all cells)
   float DXf, flf;         // DX and froude_limit as floats (estimates only)
   float act_hi, act_lo;   // (float)(active*1.5), (float)(active/4): sort_active's estimates
-  long long thr_key;      // dkey(hflow_threshold)
+  long long thr_key, thr_xkey;  // dkey, xkey(hflow_threshold) (xkey of +0 for a zero)
   int imax, jmax;
   size_t W, N2, E2;       // pitch, padded cells, edge-array cells
 
@@ -407,6 +407,13 @@ HC_DEV long long dkey(double x) {
   const long long s = b >> 63;
   return ((b & 0x7fffffffffffffffLL) ^ s) - s;
 }
+// the same order in three instructions instead of five, but for -0 < +0:
+// where the sign of a zero cannot matter
+HC_DEV long long xkey(double x) {
+  const long long b = dbits(x);
+  return b ^ ((b >> 63) & 0x7fffffffffffffffLL);
+}
+constexpr long long kNoDataXKey = -0x40C3878000000001LL;  // xkey(-9999.0)
 HC_DEV bool dgt0(double x) { return dbits(x) > 0; }                     // x > 0
 HC_DEV bool dlt0(double x) { return dbits(x) < 0 && (dbits(x) << 1) != 0; }  // x < 0
 HC_DEV bool deq0(double x) { return (dbits(x) << 1) == 0; }             // x == 0
@@ -414,6 +421,8 @@ HC_DEV bool dlt(double a, double b) { return dkey(a) < dkey(b); }       // a < b
 HC_DEV bool dgt(double a, double b) { return dkey(a) > dkey(b); }       // a > b
 constexpr long long kNoDataKey = -0x40C3878000000000LL;  // dkey(-9999.0)
 constexpr long long kNoDataBits = (long long)0xC0C3878000000000ULL;  // dbits(-9999.0)
+// the larger of two values; of two zeros, either
+HC_DEV double xmax_d(double a, double b) { return xkey(a) < xkey(b) ? b : a; }
 // smax on the integer pipe
 HC_DEV double imax_d(double a, double b) { return dlt(a, b) ? b : a; }
 // 0 - x (the reference's spelling of a negation: +0 for x = +0)
@@ -483,7 +492,8 @@ HC_DEV double icube_rn(double h) {
 // sqrt(x) rounded to nearest, on the integer pipe, for positive normal x:
 // x = m' 2^E' with E' even and m' in [2^52, 2^54); s = floor(sqrt(m' 2^52))
 // (53 bits) from a 64-bit reciprocal square root of m' (a float rsqrt.approx
-// estimate, then two Newton-Raphson steps y (3 - u y^2) / 2 in fixed point),
+// estimate, then two Newton-Raphson steps y (3 - u y^2) / 2 in fixed point
+// on 32-bit factors where the error term has no more bits),
 // settled by the exact remainder r = m' 2^52 - s^2 and rounded up when
 // r > s (a square root never falls on a midpoint).  Other x take the
 // hardware square root through a call (kept out of line so that its FP64
@@ -504,16 +514,25 @@ HC_DEV double isqrt_rn(double x) {
       __uint_as_float((unsigned)((127 + big) << 23) | (unsigned)((mp >> (29 + big)) & 0x7fffffu));
   float r0;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(uf));
-  const unsigned rb = __float_as_uint(r0);  // r0 in (0.5, 1]
-  unsigned long long Y = (unsigned long long)((rb & 0x7fffffu) | 0x800000u) << ((int)(rb >> 23) - 87);
-#pragma unroll
-  for (int k = 0; k < 2; k++) {  // Y ~ 2^63 / sqrt(m' / 2^52)
-    const unsigned long long P_hi = __umul64hi(Y, Y);
-    const unsigned long long W = (unsigned long long)(((u128)mp * P_hi) >> 52);  // ~2^62 u y^2
-    const long long E0 = (long long)((1ull << 62) - W);  // ~2^62 (1 - u y^2), small
-    const unsigned long long aE = (E0 < 0) ? (unsigned long long)(-E0) : (unsigned long long)E0;
-    const unsigned long long c = (unsigned long long)(((u128)Y * aE) >> 63);  // Y |E0| / 2^63
-    Y = (E0 < 0) ? Y - c : Y + c;
+  const uint32_t rb = __float_as_uint(r0);  // r0 in (0.5, 1]
+  const uint32_t Y0 = min(((rb & 0x7fffffu) | 0x800000u) << ((int)(rb >> 23) - 119), 0x7fffffffu);
+  // Y ~ 2^63 / sqrt(m' / 2^52): the steps add Y E / 2^63, E = 2^62 (1 - u y^2)
+  // in units of one.  |E| is below 2^42 in the first, where Y has 31 bits,
+  // and below 2^22 in the second, so 32-bit factors carry them.
+  const uint32_t ml = (uint32_t)mp, mh = (uint32_t)(mp >> 32);
+  unsigned long long P = (unsigned long long)Y0 * Y0;  // Y^2 / 2^64
+  const long long E1 = (long long)((1ull << 62) - (unsigned long long)(((u128)mp * P) >> 52));
+  unsigned long long Y = ((unsigned long long)Y0 << 32) +
+                         (unsigned long long)(((long long)(int)Y0 * (int)(E1 >> 11)) >> 20);
+  P = __umul64hi(Y, Y);
+  {
+    const uint32_t Pl = (uint32_t)P, Ph = (uint32_t)(P >> 32);
+    const unsigned long long p0 = (unsigned long long)ml * Pl;
+    const unsigned long long p1 = (unsigned long long)ml * Ph + (p0 >> 32);
+    const unsigned long long p2 = (unsigned long long)mh * Pl + (uint32_t)p1;
+    const uint32_t w2 = mh * Ph + (uint32_t)(p1 >> 32) + (uint32_t)(p2 >> 32);
+    const int E2 = -(int)__funnelshift_r((uint32_t)p2, w2, 20);  // bits 52..83
+    Y += (unsigned long long)(((long long)(unsigned long long)(Y >> 32) * E2) >> 31);
   }
   unsigned long long s = (unsigned long long)(((u128)mp * Y) >> 63);
   long long r = (long long)((mp << 52) - s * s);  // exact: |r| < 2^63
@@ -677,16 +696,15 @@ HC_DEV float d2f_i(double x) {
   return __uint_as_float(sgn | (e << 23) | m);
 }
 
-// A float within a relative 2^-20 of |x| (or 0 / +inf when |x| is outside
-// the float normal range), built with integer operations only: the FP64
+// A float within a relative 2^-20 of |x| (or below 2^-126 / +inf when |x| is
+// outside the float normal range), built with integer operations only: the FP64
 // pipe is the scarce resource on this GPU, and these estimates only decide
 // which side of a threshold a value lies on (see near_or_above).
 HC_DEV float approx_abs_f(double x) {
-  const int hi = __double2hiint(x);
-  const int e = ((hi >> 20) & 0x7ff) - 1023 + 127;
-  if (e <= 0) return 0.0f;
-  if (e >= 255) return __int_as_float(0x7f800000);
-  return __int_as_float((e << 23) | ((hi & 0xfffff) << 3));
+  // the float's exponent and top mantissa bits are the double's, rebiased;
+  // clamped to [0, inf] (values below the normal range come out subnormal)
+  const int u = (__double2hiint(x) & 0x7fffffff) - ((1023 - 127) << 20);
+  return __int_as_float(min(max(u, 0), 0xff << 20) << 3);
 }
 
 // Signed variant of approx_abs_f.
