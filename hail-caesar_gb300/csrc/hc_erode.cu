@@ -684,7 +684,7 @@ __global__ void __launch_bounds__(256) k_apply_gather(const hc_view c, hc_dev* d
 
 // Chains are walked by one thread each when there are many (all of them in
 // flight at once), by one warp each when there are few (each one faster).
-// With many, a thread walks the first kHandOff rows of its chain and hands a
+// With many, a thread walks the first rows of its chain and hands a
 // longer chain to the warp walkers: the rows it holds go back to memory and
 // the rest of the chain is listed as a resume point (bit 31: the row before
 // it is part of the chain).
@@ -696,7 +696,17 @@ static unsigned walk_blocks(size_t N2) {
   return (unsigned)std::min<size_t>(152 * 8, std::max<size_t>(16, N2 / 2048));
 }
 __device__ __forceinline__ unsigned warps_in_flight() { return gridDim.x * (blockDim.x >> 5); }
-constexpr int kHandOff = 32;
+// How many rows that is goes by the chains there are per resident thread (two
+// blocks of a multiprocessor): while each thread walks several, a long one
+// costs its warp little, but with one or two apiece the launch lasts as long
+// as its longest walk.  16 rows, and two more per chain a thread gets, up to
+// 32 (us an iteration at 16, 24, 32 rows: 369, 377, 388 at 600^2 with less
+// than one chain a thread, 665, 658, 673 at 1000^2 with two, 2274, 2161, 2147
+// at 2000^2 with eight).
+__device__ __forceinline__ int hand_off(unsigned nch) {
+  const unsigned lanes = min(gridDim.x, 2u * 152u) * blockDim.x;
+  return 16 + 2 * (int)min(nch / lanes, 8u);
+}
 constexpr uint32_t kResumeU = 0x80000000u;
 
 // A row's inputs to the walkers, staged in shared memory by asynchronous
@@ -787,6 +797,7 @@ __global__ void __launch_bounds__(128) k_apply_xchains_t(const hc_view c, hc_dev
   if (d->xchains <= warps_in_flight()) return;  // few chains: the warp walker takes them
   StagedRow* st = &slots[threadIdx.x];
   const unsigned nch = d->xchains;
+  const int most = hand_off(nch);
   const double mult = d->mult, ts = d->s.time_step;
   const double thr = c.p.water_depth_erosion_threshold;
   const size_t W = c.W;
@@ -846,7 +857,7 @@ __global__ void __launch_bounds__(128) k_apply_xchains_t(const hc_view c, hc_dev
       live = false;
       continue;
     }
-    if (++steps >= kHandOff) {  // a long chain: the warp walkers go on from row r+1
+    if (++steps >= most) {  // a long chain: the warp walkers go on from row r+1
       row_store(c, cell, C);
       row_store(c, dcell, D);
       cp_async_wait_all();
@@ -879,6 +890,7 @@ __global__ void __launch_bounds__(128) k_apply_ychains_t(const hc_view c, hc_dev
   if (d->ychains <= warps_in_flight()) return;
   StagedRow* st = &slots[threadIdx.x];
   const unsigned nch = d->ychains;
+  const int most = hand_off(nch);
   const double mult = d->mult, ts = d->s.time_step;
   const size_t W = c.W;
   auto lat = [&](int qq, bool m, double et3) { return qq >= 2 && qq <= c.jmax - 1 && m && dgt0(et3); };
@@ -930,7 +942,7 @@ __global__ void __launch_bounds__(128) k_apply_ychains_t(const hc_view c, hc_dev
       live = false;
       continue;
     }
-    if (++steps >= kHandOff) {  // a long chain: the warp walkers go on from column q+1
+    if (++steps >= most) {  // a long chain: the warp walkers go on from column q+1
       row_store(c, cell, C);
       row_store(c, dcell, D);
       cp_async_wait_all();
