@@ -399,8 +399,6 @@ static hc_status free_all(hc_ctx* c) {
   sort_work_free(c->sort_work);
   free(extra(c).h_rain);
   if (c->graph) cudaGraphExecDestroy(c->graph);
-  for (auto& t : c->tail)
-    if (t) cudaGraphExecDestroy(t);
   if (c->chunk_done) cudaEventDestroy(c->chunk_done);
   if (c->s) cudaStreamDestroy(c->s);
   if (c->s2) cudaStreamDestroy(c->s2);
@@ -1090,7 +1088,9 @@ static hc_status capture_iteration(hc_ctx* c, int flags) {
   cudaGraph_t cg;
   HC_CU(cudaStreamGetCaptureInfo(c->s, &st, nullptr, &cg, nullptr, nullptr, nullptr), "capture info");
   hc_iter_handles& H = c->hcur;
+  const cudaGraphConditionalHandle loop = H.loop;
   std::memset(&H, 0, sizeof H);
+  H.loop = loop;
   const bool sed = !c->v.p.hydro_only;
   auto mk = [&](cudaGraphConditionalHandle* h) {
     return cudaGraphConditionalHandleCreate(h, cg, 0, cudaGraphCondAssignDefault);
@@ -1128,68 +1128,69 @@ static hc_status capture_iteration(hc_ctx* c, int flags) {
   return HC_OK;
 }
 
-// iterations per chunk graph: HC_GRAPH_ITERS if set, else what the caller
-// asked for (hc_run_ensemble: 128), else 32
-static int graph_chunk(const hc_ctx* c) {
+// iterations in the loop's body: HC_GRAPH_ITERS if set, else one
+static int graph_body() {
   const char* e = getenv("HC_GRAPH_ITERS");
-  int k = e ? atoi(e) : (c->chunk_pref > 0 ? c->chunk_pref : 32);
-  return std::max(1, std::min(k, 4096));
+  return std::max(1, std::min(e ? atoi(e) : 1, 4096));
 }
 
-// Captures K iterations into *exec; *kernels = kernel nodes outside
-// conditional bodies (they run on every launch; those inside run only when
-// their condition is set, and the device counts them).
-static hc_status build_one(hc_ctx* c, int flags, int K, cudaGraphExec_t* exec,
-                           int64_t* kernels) {
-  if (*exec) cudaGraphExecDestroy(*exec);
-  *exec = nullptr;
+// The graph of a run: a WHILE node that repeats one iteration until the
+// device finds a reason to stop (the budget is spent, the host has work to
+// do, the run's end).  k_control and k_flux_out set its condition.
+//
+// Before, graphs of 32 (ensembles: 128) and of 16, 8, 4, 2 and 1 iterations
+// were captured and instantiated whenever flags, launch shape or record
+// buffer changed, and a launch skipped the iterations left after a pause.
+// The first run of twelve members after a shape change took 1.2 s, now 69 ms;
+// an iteration of a 128 x 128 catchment 169 us, now 144; of the 300 x 100
+// reach 279, now 261.  Bodies of 2, 4 or 8 iterations are at most 2 % faster
+// (257 us, the reach) and skip iterations at a run's end.
+static hc_status build_graph(hc_ctx* c, int flags) {
+  const int K = graph_body();
+  if (c->graph) cudaGraphExecDestroy(c->graph);
+  c->graph = nullptr;
+  c->graph_iters = 0;
   cudaGraph_t g;
-  HC_CU(cudaStreamBeginCapture(c->s, cudaStreamCaptureModeRelaxed), "capture");
+  HC_CU(cudaGraphCreate(&g, 0), "graph");
+  struct Drop {
+    cudaGraph_t g;
+    ~Drop() { cudaGraphDestroy(g); }
+  } drop{g};
+  std::memset(&c->hcur, 0, sizeof c->hcur);
+  HC_CU(cudaGraphConditionalHandleCreate(&c->hcur.loop, g, 1, cudaGraphCondAssignDefault),
+        "handle");
+  cudaGraphNodeParams prm = {};
+  prm.type = cudaGraphNodeTypeConditional;
+  prm.conditional.handle = c->hcur.loop;
+  prm.conditional.type = cudaGraphCondTypeWhile;
+  prm.conditional.size = 1;
+  cudaGraphNode_t node;
+  HC_CU(cudaGraphAddNode(&node, g, nullptr, nullptr, 0, &prm), "loop node");
+  cudaGraph_t body = prm.conditional.phGraph_out[0];
+  HC_CU(cudaStreamBeginCaptureToGraph(c->s, body, nullptr, nullptr, 0,
+                                      cudaStreamCaptureModeRelaxed), "capture");
   c->capturing = true;
   hc_status cst = HC_OK;
   for (int k = 0; k < K && cst == HC_OK; k++) cst = capture_iteration(c, flags);
   c->capturing = false;
   c->cs = c->s;
   std::memset(&c->hcur, 0, sizeof c->hcur);
-  cudaError_t ee = cudaStreamEndCapture(c->s, &g);
-  if (cst != HC_OK) {
-    if (ee == cudaSuccess) cudaGraphDestroy(g);
-    return cst;
-  }
+  cudaGraph_t out;
+  const cudaError_t ee = cudaStreamEndCapture(c->s, &out);
+  HC_TRY(cst);
   HC_CU(ee, "capture");
   size_t nn = 0;
-  cudaGraphGetNodes(g, nullptr, &nn);
+  cudaGraphGetNodes(body, nullptr, &nn);
   std::vector<cudaGraphNode_t> nodes(nn);
-  cudaGraphGetNodes(g, nodes.data(), &nn);
-  *kernels = 0;
+  cudaGraphGetNodes(body, nodes.data(), &nn);
+  c->graph_kernels = 0;
   for (auto nd : nodes) {
     cudaGraphNodeType t;
     cudaGraphNodeGetType(nd, &t);
-    if (t == cudaGraphNodeTypeKernel) (*kernels)++;
+    if (t == cudaGraphNodeTypeKernel) c->graph_kernels++;
   }
-  cudaError_t e = cudaGraphInstantiate(exec, g, 0);
-  cudaGraphDestroy(g);
-  HC_CU(e, "graph instantiate");
-  return HC_OK;
-}
-
-// The chunk graph (K iterations) and, for runs shorter than K, the graphs of
-// 2^k < K iterations (a paused chunk skips the rest of its iterations, so a
-// short run would otherwise pay for K).  All are made and uploaded here, so
-// that no later hc_run instantiates a graph between its launches.
-static hc_status build_graph(hc_ctx* c, int flags) {
-  const int K = graph_chunk(c);
-  for (auto& t : c->tail)
-    if (t) {
-      cudaGraphExecDestroy(t);
-      t = nullptr;
-    }
-  HC_TRY(build_one(c, flags, K, &c->graph, &c->graph_kernels));
+  HC_CU(cudaGraphInstantiate(&c->graph, g, 0), "graph instantiate");
   HC_CU(cudaGraphUpload(c->graph, c->s), "graph upload");
-  for (int k = 0; k < 12 && (1 << k) < K; k++) {
-    HC_TRY(build_one(c, flags, 1 << k, &c->tail[k], &c->tail_kernels[k]));
-    HC_CU(cudaGraphUpload(c->tail[k], c->s), "graph upload");
-  }
   c->graph_iters = K;
   c->graph_flags = flags;
   return HC_OK;
@@ -1304,43 +1305,35 @@ static hc_status run_begin(hc_ctx* c, int64_t n, int32_t flags, bool want_rec, b
     HC_TRY(pull(c));
   }
   HC_TRY(autotune(c, false));  // launch shapes for this shape class (hc_tune.cu)
-  if (!c->graph_iters || c->graph_flags != flags || c->graph_iters != graph_chunk(c))
+  if (!c->graph_iters || c->graph_flags != flags || c->graph_iters != graph_body())
     HC_TRY(build_graph(c, flags));
   if (!c->chunk_done) HC_CU(cudaEventCreateWithFlags(&c->chunk_done, cudaEventDisableTiming),
                             "event");
   return HC_OK;
 }
 
-// one graph chunk, then the control block copied back; chunk_done marks both
+// the graph, then the control block copied back; chunk_done marks both
 static hc_status run_launch(hc_ctx* c) {
   c->body_k0 = c->hdev->body_kernels;
   c->budget0 = c->hdev->budget;
   c->stat_n[HC_STAT_CHUNKS]++;
-  if (c->budget0 >= c->graph_iters) {
-    c->chunk_iters = c->graph_iters;
-    HC_CU(cudaGraphLaunch(c->graph, c->s), "graph launch");
-    c->launches += c->graph_kernels;
-  } else {
-    int k = 0;
-    while (k + 1 < 12 && (2LL << k) <= c->budget0) k++;
-    if (!c->tail[k]) HC_TRY(build_one(c, c->graph_flags, 1 << k, &c->tail[k], &c->tail_kernels[k]));
-    c->chunk_iters = 1 << k;
-    HC_CU(cudaGraphLaunch(c->tail[k], c->s), "graph launch");
-    c->launches += c->tail_kernels[k];
-  }
+  HC_CU(cudaGraphLaunch(c->graph, c->s), "graph launch");
   c->d2h_bytes += sizeof(hc_dev);
   HC_CU(cudaMemcpyAsync(c->hdev, c->dev, sizeof(hc_dev), cudaMemcpyDeviceToHost, c->s), "pull");
   HC_CU(cudaEventRecord(c->chunk_done, c->s), "event");
   return HC_OK;
 }
 
-// after a chunk: host-side work the device asked for; *finished when done
+// after a launch: host-side work the device asked for; *finished when done
 static hc_status run_after_chunk(hc_ctx* c, int32_t flags, bool* finished) {
   hc_dev* hd = c->hdev;
   *finished = false;
-  c->launches += (int64_t)(hd->body_kernels - c->body_k0);
-  c->stat_n[HC_STAT_IDLE_ITERS] += std::max<int64_t>(
-      0, std::min<int64_t>(c->chunk_iters, c->budget0) - (c->budget0 - hd->budget));
+  // kernels of the iterations run (the last turn of a longer body may hold
+  // skipped ones), and those of the IF nodes, which the device counts
+  const int64_t its = c->budget0 - hd->budget, K = c->graph_iters;
+  const int64_t turns = std::max<int64_t>(1, (its + K - 1) / K);
+  c->launches += turns * c->graph_kernels + (int64_t)(hd->body_kernels - c->body_k0);
+  c->stat_n[HC_STAT_IDLE_ITERS] += turns * K - its;
   if (hd->pause & HC_PAUSE_ERROR) return device_error(c);
   if (hd->pause & (HC_PAUSE_ERODE | HC_PAUSE_LATERAL)) HC_TRY(finish_iteration(c, flags));
   HC_TRY(host_steps(c, flags));
@@ -1385,9 +1378,8 @@ extern "C" hc_status hc_run(hc_ctx* c, int64_t n, int32_t flags, hc_step_record*
   return run_end(c, rec, done);
 }
 
-// The service loop of a group of members: launch each member's first chunk,
-// then, whichever member's chunk has finished, do its host work and launch
-// its next chunk.
+// The service loop of a group of members: launch each member's graph, then,
+// whichever member's graph has stopped, do its host work and launch it again.
 static hc_status ensemble_group(hc_ctx** ctxs, const std::vector<int>& mine, int64_t n,
                                 int32_t flags, int64_t* done) {
   std::vector<char> live(mine.size(), 0);
@@ -1430,7 +1422,7 @@ static hc_status ensemble_group(hc_ctx** ctxs, const std::vector<int>& mine, int
 // Members are shared out over host threads (member k to thread k mod T), so
 // that one member's host work (a drainage recomputation, the daily global
 // landsliding, lateral3's convergence loop) holds up only the members of its
-// own thread while the device runs the others' chunks.
+// own thread while the device runs the others' graphs.
 extern "C" hc_status hc_run_ensemble(hc_ctx** ctxs, int32_t m, int64_t n, int32_t flags,
                                      int64_t* done) {
   if (!ctxs || m <= 0 || n < 0) return HC_ERR_ARG;
@@ -1438,8 +1430,6 @@ extern "C" hc_status hc_run_ensemble(hc_ctx** ctxs, int32_t m, int64_t n, int32_
     if (!ctxs[k]) return HC_ERR_ARG;
     if (done) done[k] = 0;
   }
-  // longer chunks: fewer host turns per member while the others run
-  for (int k = 0; k < m; k++) ctxs[k]->chunk_pref = 128;
   const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
   const int T = (int)std::max(1u, std::min<unsigned>((unsigned)m, std::min(hw, 32u)));
   std::vector<std::vector<int>> groups((size_t)T);

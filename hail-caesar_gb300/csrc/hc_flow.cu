@@ -115,6 +115,14 @@ __global__ void __launch_bounds__(32) k_control(const hc_view c, hc_dev* d, hc_i
     if (l0) {
       if (budget <= 0) d->pause = pause | HC_PAUSE_BUDGET;
       d->it_active = 0;
+      if (hh.has) {  // no step of it runs, and no iteration follows
+        cudaGraphSetConditional(hh.loop, 0u);
+        cudaGraphSetConditional(hh.scan, 0u);
+        if (!p.hydro_only)
+          for (const cudaGraphConditionalHandle h :
+               {hh.erode, hh.retry2, hh.retry3, hh.retry4, hh.erode_fin, hh.slide})
+            cudaGraphSetConditional(h, 0u);
+      }
     }
     return;
   }
@@ -332,8 +340,14 @@ __global__ void __launch_bounds__(32) k_control(const hc_view c, hc_dev* d, hc_i
   if (hh.has) {
     // kernels inside the bodies enabled here: scan 3, erosion 5 + 7, slide_3 4
     d->body_kernels += (scan ? 3 : 0) + (erode ? 12 : 0) + (slide ? 4 : 0);
+    // the loop goes on when water_flux_out says so; an iteration that stops
+    // before it ends the loop
+    cudaGraphSetConditional(hh.loop, 0u);
     cudaGraphSetConditional(hh.scan, scan ? 1u : 0u);
     if (!p.hydro_only) {
+      cudaGraphSetConditional(hh.retry2, 0u);
+      cudaGraphSetConditional(hh.retry3, 0u);
+      cudaGraphSetConditional(hh.retry4, 0u);
       cudaGraphSetConditional(hh.erode, erode ? 1u : 0u);
       cudaGraphSetConditional(hh.erode_fin, erode ? 1u : 0u);
       cudaGraphSetConditional(hh.slide, slide ? 1u : 0u);
@@ -1025,7 +1039,8 @@ __global__ void __launch_bounds__(1024) k_wet_write(const hc_view c, const hc_de
 constexpr int kFluxSums = 1024, kFluxThreads = 512;
 
 __global__ void __launch_bounds__(kFluxThreads) k_flux_out(const hc_view c, hc_dev* d, int gated, int record,
-                                                   hc_step_record* rec, int64_t rec_cap) {
+                                                   hc_step_record* rec, int64_t rec_cap,
+                                                   cudaGraphConditionalHandle loop, int has_loop) {
   __shared__ double part[kFluxSums];
   __shared__ double vpart[kFluxSums];
   if (gated && !(d->it_active && d->rest_active)) return;
@@ -1167,6 +1182,7 @@ __global__ void __launch_bounds__(kFluxThreads) k_flux_out(const hc_view c, hc_d
       if (!p.hydro_only && !(d->flags & HC_RUN_NOHILL) && (r.cycle > creep1 || r.cycle > creep2))
         d->pause |= HC_PAUSE_HOSTSTEP;
       if (!(r.cycle / 60 < p.maxcycle)) d->pause |= HC_PAUSE_FINISHED;
+      if (has_loop) cudaGraphSetConditional(loop, d->pause == 0 && d->budget > 0 ? 1u : 0u);
     }
   }
 }
@@ -1309,7 +1325,7 @@ void launch_flux_out(hc_ctx* c, int gated, int record) {
   // memory then, and no block waits for another's arrival
   const int blocks = n <= kFluxSums ? 1 : std::min((n + kFluxThreads - 1) / kFluxThreads, 64);
   k_flux_out<<<blocks, kFluxThreads, 0, c->cs>>>(c->v, c->dev, gated, record, c->v.rec,
-                                                 c->v.rec_cap);
+                                                 c->v.rec_cap, c->hcur.loop, c->capturing ? 1 : 0);
   count_launch(c, 1);
 }
 

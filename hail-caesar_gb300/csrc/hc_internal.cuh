@@ -217,6 +217,7 @@ struct hc_view {
 // not due this iteration are not launched at all.
 struct hc_iter_handles {
   cudaGraphConditionalHandle scan, erode, retry2, retry3, retry4, erode_fin, slide;
+  cudaGraphConditionalHandle loop;  // the run's WHILE node: another iteration
   int has;  // 0 outside graph capture: nothing to set
 };
 
@@ -252,19 +253,14 @@ struct hc_ctx {
   // called after every recomputation of the input points (adjoint replays)
   void (*points_hook)(hc_ctx*, void*);
   void* points_hook_arg;
-  // CUDA graph of K iterations
+  // CUDA graph of a run: a WHILE node whose body is one iteration (or
+  // graph_iters of them); graph_iters 0: to be built
   cudaGraphExec_t graph; int graph_iters; int graph_flags;
-  int64_t graph_kernels;   // kernel nodes in the graph
-  // graphs of 2^k iterations (k < 12) for runs shorter than a chunk, made
-  // when first needed: a short run takes the fewest launches (20 = 16 + 4)
-  cudaGraphExec_t tail[12];
-  int64_t tail_kernels[12];
-  int chunk_pref;          // iterations per chunk graph asked for (0: the default)
-  int chunk_iters;         // iterations in the chunk last launched
-  cudaEvent_t chunk_done;  // a launched chunk and its control-block copy are done
+  int64_t graph_kernels;   // kernel nodes in the body outside its IF nodes
+  cudaEvent_t chunk_done;  // a launched graph and its control-block copy are done
   int64_t run_n;           // iterations asked of the current run
   unsigned long long body_k0;
-  int64_t budget0;         // budget when the current chunk was launched
+  int64_t budget0;         // budget when the graph was last launched
   bool capturing;
   // counters for measurement: kernels launched, bytes moved host<->device
   int64_t launches, h2d_bytes, d2h_bytes;

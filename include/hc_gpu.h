@@ -361,8 +361,9 @@ hc_status hc_adj_gradient(hc_ctx* ctx, int64_t n, int32_t max_states, const doub
 
 /* What hc_run spent on the host (no counterpart in the reference): for
  * each kind below, how many times it ran and its host wall time in ms,
- * accumulated since hc_create.  Pauses leave the rest of a graph chunk as
- * no-op iterations; HC_STAT_IDLE_ITERS counts those. */
+ * accumulated since hc_create.  A run's graph repeats one iteration until
+ * the device stops it; where a body of more iterations was asked for
+ * (HC_GRAPH_ITERS), HC_STAT_IDLE_ITERS counts those skipped after a stop. */
 enum {
   HC_STAT_CHUNKS = 0,      /* graph launches */
   HC_STAT_ERODE_RETRY,     /* erosion retries past the captured passes */
