@@ -248,6 +248,7 @@ extern "C" hc_status hc_create(const hc_params* p, size_t max_bytes, hc_ctx** ou
   v.rDX = 1.0 / p->DX;
   v.dxd = host_divisor(p->DX);
   v.fived = host_divisor(5.0);
+  v.diagd = host_divisor(1.414);
   v.nn = p->mannings * p->mannings;
   v.DXf = (float)p->DX;
   v.flf = (float)p->froude_limit;
@@ -859,30 +860,24 @@ extern "C" hc_status hc_prepare(hc_ctx* c) {
   if (!x.h_rain) return hc_fail(c, HC_ERR_STATE, "hc_set_rain must come before hc_prepare");
   for (int n = 0; n < p.number_of_points && p.reach_mode; n++)
     if (!v.reach[n]) return hc_fail(c, HC_ERR_STATE, "reach table %d missing", n);
-  const size_t N2 = v.N2;
-  std::vector<double> elev(N2);
-  std::vector<int32_t> rf(N2);
-  HC_CU(cudaStreamSynchronize(c->s), "prepare");
-  HC_CU(cudaMemcpy(elev.data(), v.elev, N2 * 8, cudaMemcpyDeviceToHost), "prepare");
-  HC_CU(cudaMemcpy(rf.data(), v.rfarea, N2 * 4, cudaMemcpyDeviceToHost), "prepare");
   HC_TRY(pull(c));
   hc_scalars& s = c->hdev->s;
-  for (int n = 0; n <= HC_MAX_RF; n++) s.nActualGridCells[n] = 0;
-  for (int i = 1; i < p.imax; i++)  // count_catchment_gridcells :2813 (i < imax, j < jmax)
-    for (int j = 1; j < p.jmax; j++)
-      if (elev[(size_t)i * v.W + j] > -9999) {
-        const int r = rf[(size_t)i * v.W + j];
-        if (r < 0 || r > p.rfnum) return hc_fail(c, HC_ERR_ARG, "rfarea value %d out of range", r);
-        s.nActualGridCells[r] += 1;
-      }
+  {
+    bool ok = true;
+    int r = 0;
+    HC_TRY(count_zone_cells(c, s.nActualGridCells, &ok, &r));
+    if (!ok) return hc_fail(c, HC_ERR_ARG, "rfarea value %d out of range", r);
+  }
   s.creep_time = s.creep_time2 = s.time_1 = s.cycle;  // set_time_counters :1862
   // TOPMODEL rows: initialise_rainfall_runoff's call, then one per minute
   const int rows = p.maxcycle * 60 + std::max(0, p.max_time_step / 60) + 2000;
   std::vector<double> table((size_t)rows * 2 * (p.rfnum + 1));
   host_topmodel_table(&p, x.h_rain, x.h_rain_rows, x.h_rain_cols, rows, table.data());
-  if (v.topm) cudaFree(v.topm);
-  v.topm = nullptr;
-  HC_TRY(dalloc(c, &v.topm, table.size()));
+  if (!v.topm || v.topm_rows != rows) {  // a repeated set-up keeps its table's memory
+    if (v.topm) cudaFree(v.topm);
+    v.topm = nullptr;
+    HC_TRY(dalloc(c, &v.topm, table.size()));
+  }
   HC_CU(cudaMemcpy(v.topm, table.data(), table.size() * 8, cudaMemcpyHostToDevice), "prepare");
   v.topm_rows = rows;
   for (int n = p.spatially_complex_rainfall ? 0 : 1; n <= p.rfnum; n++) {
@@ -896,15 +891,12 @@ extern "C" hc_status hc_prepare(hc_ctx* c) {
     // skips the drainage area and the input points in this mode (:2055-2070)
     for (int z = 0; z <= HC_MAX_RF; z++) v.runoff_count[z] = 0;
     v.runoff_present = 0;
-    for (int i = 1; i < p.imax; i++)
-      for (int j = 1; j < p.jmax; j++) {
-        const size_t cell = (size_t)i * v.W + j;
-        if (!(elev[cell] > -9999)) continue;
-        const int r = rf[cell];
-        const int z = (p.rfnum == 1) ? 1 : ((r >= 1 && r <= p.rfnum - 1) ? r : 0);
-        v.runoff_count[z] += 1;
-        v.runoff_present |= 1u << z;
-      }
+    for (int r = 0; r <= p.rfnum; r++) {
+      if (!(s.nActualGridCells[r] > 0)) continue;
+      const int z = (p.rfnum == 1) ? 1 : ((r >= 1 && r <= p.rfnum - 1) ? r : 0);
+      v.runoff_count[z] += s.nActualGridCells[r];
+      v.runoff_present |= 1u << z;
+    }
     HC_TRY(push(c));
   } else {
     HC_TRY(push(c));

@@ -107,26 +107,36 @@ __global__ void k_sel_hist(const hc_view c, const double* __restrict__ el, int s
     if (h[k]) atomicAdd(&c.drain_aux->hist[k], h[k]);
 }
 
-__global__ void k_sel_pick(const hc_view c, int shift, unsigned long long padding) {
+// one block of 256 threads, a digit each: the suffix sums of the counts, then
+// the digit whose sum is the first to reach k
+__global__ void __launch_bounds__(256) k_sel_pick(const hc_view c, int shift,
+                                                  unsigned long long padding) {
+  __shared__ unsigned long long sum[256];
   hc_drain_aux* a = c.drain_aux;
+  const int d = threadIdx.x;
   const unsigned long long zero_digit = (kZeroKey >> shift) & 255;
   const bool zero_in = (kZeroKey & a->mask) == a->prefix;
-  unsigned long long cum = 0;
-  int digit = 0;
-  for (int d = 255; d >= 0; d--) {
-    const unsigned long long n = a->hist[d] + ((zero_in && (unsigned)d == zero_digit) ? padding : 0);
-    if (cum + n >= a->k) {
-      digit = d;
-      a->real_eq = a->hist[d];
-      break;
-    }
-    cum += n;
+  const unsigned long long k = a->k;
+  const unsigned real = a->hist[d];
+  const unsigned long long n = real + ((zero_in && (unsigned)d == zero_digit) ? padding : 0);
+  sum[d] = n;
+  __syncthreads();
+  for (int o = 1; o < 256; o <<= 1) {
+    const unsigned long long v = d + o < 256 ? sum[d + o] : 0;
+    __syncthreads();
+    sum[d] += v;
+    __syncthreads();
   }
-  a->k -= cum;
-  a->gt += cum;
-  a->prefix |= (unsigned long long)digit << shift;
-  a->mask |= 255ull << shift;
-  for (int d = 0; d < 256; d++) a->hist[d] = 0;
+  const unsigned long long above = sum[d] - n;  // keys with a larger digit
+  // k is at most the number of keys left, so one digit takes it
+  if (above < k && sum[d] >= k) {
+    a->real_eq = real;
+    a->k = k - above;
+    a->gt += above;
+    a->prefix |= (unsigned long long)d << shift;
+    a->mask |= 255ull << shift;
+  }
+  a->hist[d] = 0;
 }
 
 // sorted position of every cell the sweep reaches (1 .. imax*jmax); 0 = not
@@ -159,7 +169,7 @@ __global__ void k_drain_init(const hc_view c, hc_dev* d, const double* __restric
     if (dir % 2 != 0) {
       if (e2 < e) difftot += e - e2;
     } else {
-      if (e2 < e) difftot += (e - e2) / 1.414;
+      if (e2 < e) difftot += ddiv_by(e - e2, c.diagd);
     }
   }
   c.drain_dt[cell] = difftot;
@@ -212,54 +222,70 @@ __global__ void k_drain_init(const hc_view c, hc_dev* d, const double* __restric
 // own unit of area counts (not no-data).
 constexpr int kHeadCount = 32, kHeadLower = 36, kHeadReached = 45, kHeadOwn = 46;
 
-__global__ void k_drain_terms(const hc_view c, const double* __restrict__ el) {
+// Elevations are compared as integer keys (a NaN, below and above nothing, as
+// the cell's own key), and quotients run on the integer pipe: a pick of the
+// next higher neighbour is up to nine compares, which as FP64 instructions
+// took most of the kernel's time: 1912 -> 232 us at 1500^2.
+__global__ void __launch_bounds__(256) k_drain_terms(const hc_view c,
+                                                     const double* __restrict__ el) {
   int i, j;
   if (!interior_ij(c, i, j)) return;
   const size_t W = c.W;
   const size_t cell = (size_t)i * W + j;
   const double e = el[cell];
+  const long long ke = dkey(e);
   unsigned left = 0, lower = 0;
-  double en[9];
+  long long kn[9];
   uint32_t pn[9];
 #pragma unroll
   for (int k = 0; k < 9; k++) {
     const int iq = i + k / 3 - 1, jq = j + k % 3 - 1;
     const bool in = k != 4 && iq >= 1 && iq <= c.imax && jq >= 1 && jq <= c.jmax;
     const size_t q = (size_t)iq * W + jq;
-    en[k] = in ? el[q] : e;
+    const double en = in ? el[q] : e;
+    kn[k] = disnan(en) || disnan(e) ? ke : dkey(en);
     pn[k] = in ? c.drain_pos[q] : 0u;
-    if (en[k] > e && pn[k] != 0) left |= 1u << k;
-    if (en[k] < e) lower |= 1u << k;
+    if (kn[k] > ke && pn[k] != 0) left |= 1u << k;
+    if (kn[k] < ke) lower |= 1u << k;
   }
   const bool reached = c.drain_pos[cell] != 0;
   unsigned long long head = ((unsigned long long)lower << kHeadLower) |
                             ((unsigned long long)reached << kHeadReached) |
-                            ((unsigned long long)(e != -9999) << kHeadOwn);
+                            ((unsigned long long)(ke != kNoDataKey) << kHeadOwn);
   int n = 0;
   if (reached) {
     double* share = c.drain_share + cell * 8;
 #pragma unroll 1
     while (left) {
       int best = -1;
-      double be = 0;
+      long long bk = 0;
       uint32_t bp = 0;
 #pragma unroll
       for (int k = 0; k < 9; k++) {
         if (!((left >> k) & 1u)) continue;
-        if (best < 0 || en[k] > be || (en[k] == be && pn[k] > bp)) {
+        if (best < 0 || kn[k] > bk || (kn[k] == bk && pn[k] > bp)) {
           best = k;
-          be = en[k];
+          bk = kn[k];
           bp = pn[k];
         }
       }
       left &= ~(1u << best);
-      const int iq = i + best / 3 - 1, jq = j + best % 3 - 1;
-      const double dq = c.drain_dt[(size_t)iq * W + jq];
+      const int di = best / 3 - 1, dj = best - 3 * (di + 1) - 1;
+      const int iq = i + di, jq = j + dj;
+      const size_t q = (size_t)iq * W + jq;
+      const double drop = el[q] - e;
+      const double dq = c.drain_dt[q];
+      if (iq > 1 && iq < c.imax && jq > 1 && jq < c.jmax) {  // one direction of q lands here
+        share[n] = ddiv_rn(di != 0 && dj != 0 ? ddiv_by(drop, c.diagd) : drop, dq);
+        head |= (unsigned long long)best << (4 * n);
+        n++;
+        continue;
+      }
 #pragma unroll 1
       for (int dir = 1; dir <= 8; dir++) {
         const int i3 = clampi(iq + kDrX[dir], 1, c.imax), j3 = clampi(jq + kDrY[dir], 1, c.jmax);
         if (i3 != i || j3 != j) continue;
-        share[n] = (dir % 2 != 0) ? ((be - e) / dq) : (((be - e) / 1.414) / dq);
+        share[n] = ddiv_rn(dir % 2 != 0 ? drop : ddiv_by(drop, c.diagd), dq);
         head |= (unsigned long long)best << (4 * n);
         n++;
       }
@@ -611,7 +637,9 @@ __global__ void __launch_bounds__(1024) k_points_write(const hc_view c, hc_dev* 
     c.cin_x[t] = (int32_t)(k / c.W);
     c.cin_y[t] = (int32_t)(k % c.W);
     const int rf = c.rfarea[k];
-    if (rf >= 0 && rf <= HC_MAX_RF) atomicAdd(&d->drain_rf[rf], 1u);
+    const unsigned same = __match_any_sync(__activemask(), rf);  // one atomic per warp and zone
+    if (rf >= 0 && rf <= HC_MAX_RF && lane == __ffs(same) - 1)
+      atomicAdd(&d->drain_rf[rf], (unsigned)__popc(same));
   }
 }
 
@@ -628,7 +656,60 @@ __global__ void k_points_finish(const hc_view c, hc_dev* d) {
   s.totalinputpoints = (t == 0) ? 1.0 : (double)t;
 }
 
+// count_catchment_gridcells :2813: the cells of rows 1 .. imax-1, columns
+// 1 .. jmax-1 above no-data, by zone; bad: the first cell whose zone is out
+// of range
+__global__ void __launch_bounds__(256) k_zone_count(const hc_view c, unsigned int* counts,
+                                                    unsigned int* bad) {
+  __shared__ unsigned int h[HC_MAX_RF + 1];
+  for (int k = threadIdx.x; k <= HC_MAX_RF; k += blockDim.x) h[k] = 0;
+  __syncthreads();
+  const size_t n = (size_t)(c.imax - 1) * c.W;
+  for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < n;
+       k += (size_t)gridDim.x * blockDim.x) {
+    const size_t cell = c.W + k;
+    const int j = (int)(k % c.W);
+    const double e = c.elev[cell];
+    if (j < 1 || j >= c.jmax || !(e > -9999)) continue;
+    const int r = c.rfarea[cell];
+    if (r < 0 || r > c.p.rfnum) {
+      atomicMin(bad, (unsigned)cell);
+      continue;
+    }
+    const unsigned same = __match_any_sync(__activemask(), r);
+    if ((int)(threadIdx.x & 31) == __ffs(same) - 1) atomicAdd(&h[r], (unsigned)__popc(same));
+  }
+  __syncthreads();
+  for (int k = threadIdx.x; k <= HC_MAX_RF; k += blockDim.x)
+    if (h[k]) atomicAdd(&counts[k], h[k]);
+}
+
 }  // namespace
+
+// nActualGridCells per zone (HC_MAX_RF + 1 entries) by the device; *bad_zone
+// receives an out-of-range zone (of the first such cell) and *ok tells.
+hc_status count_zone_cells(hc_ctx* c, double* cells, bool* ok, int* bad_zone) {
+  unsigned int* n = (unsigned int*)c->v.drain_aux->hist;  // scratch until the next selection
+  unsigned int h[HC_MAX_RF + 2];
+  cudaStream_t s = c->s;
+  cudaError_t e = cudaMemsetAsync(n, 0, (HC_MAX_RF + 1) * 4, s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(n + HC_MAX_RF + 1, 0xff, 4, s);
+  if (e == cudaSuccess) {
+    k_zone_count<<<c->sms * 4, 256, 0, s>>>(c->v, n, n + HC_MAX_RF + 1);
+    count_launch(c, 1);
+    e = cudaMemcpyAsync(h, n, sizeof h, cudaMemcpyDeviceToHost, s);
+  }
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  if (e != cudaSuccess) return hc_cuda(c, e, "prepare");
+  c->d2h_bytes += sizeof h;
+  for (int k = 0; k <= HC_MAX_RF; k++) cells[k] = (double)h[k];
+  *ok = h[HC_MAX_RF + 1] == 0xffffffffu;
+  if (!*ok) {
+    e = cudaMemcpy(bad_zone, c->v.rfarea + h[HC_MAX_RF + 1], 4, cudaMemcpyDeviceToHost);
+    if (e != cudaSuccess) return hc_cuda(c, e, "prepare");
+  }
+  return HC_OK;
+}
 
 // The drainage area for the elevations `el` (device), then the input points.
 // `sort_order` is called, and its order used, only when the sort's order
@@ -656,7 +737,7 @@ hc_status run_drainage_device(hc_ctx* c, const double* el, bool area_valid,
     k_drain_mincount<<<g, b, 0, s>>>(v, el);
     for (int shift = 56; shift >= 0; shift -= 8) {
       k_sel_hist<<<g, b, 0, s>>>(v, el, shift);
-      k_sel_pick<<<1, 1, 0, s>>>(v, shift, P);
+      k_sel_pick<<<1, 256, 0, s>>>(v, shift, P);
     }
     k_drain_init<<<g, b, 0, s>>>(v, c->dev, el);
     c->launches += 19;

@@ -132,7 +132,7 @@ struct hc_divisor {
 struct hc_view {
   hc_params p;
   double rDX;             // RN(1/DX) (the adjoint's slope derivatives)
-  hc_divisor dxd, fived;  // DX and 5 as divisors (ddiv_by)
+  hc_divisor dxd, fived, diagd;  // DX, 5 and 1.414 as divisors (ddiv_by)
   double nn;              // mannings * mannings (one n for all cells)
   float DXf, flf;         // DX and froude_limit as floats (estimates only)
   float act_hi, act_lo;   // (float)(active*1.5), (float)(active/4): sort_active's estimates
@@ -802,6 +802,7 @@ const uint32_t* host_drainage_order(const hc_params* p, const double* elev, void
                                     bool* reused);
 // sort_order(c, el, order): the sweep order for the elevations el (device)
 // into order (device, N2 entries)
+hc_status count_zone_cells(hc_ctx* c, double* cells, bool* ok, int* bad_zone);
 hc_status run_drainage_device(hc_ctx* c, const double* el, bool area_valid,
                               hc_status (*sort_order)(hc_ctx*, const double*, uint32_t*),
                               bool* sorted);
