@@ -1527,15 +1527,25 @@ void launch_erode_finish(hc_ctx* c, int gated) {
   dim3 b(32, 8);
   dim3 g((c->v.jmax - 2 + 31) / 32, (c->v.imax + 7) / 8);
   k_apply_pre<<<g, b, 0, c->cs>>>(c->v, c->dev);
+  // The edge output reads the fluxes and the suspended load as the pre-pass
+  // leaves them, which the gather and the walkers neither read nor change:
+  // in a captured iteration its one block runs beside them (an iteration of a
+  // storm: 2120 -> 1999 us at 2000^2, 357 -> 336 us at 600^2).
+  const cudaStream_t es = c->capturing ? c->side : c->cs;
+  if (c->capturing) {
+    cudaEventRecord(c->fork, c->cs);
+    cudaStreamWaitEvent(c->side, c->fork, 0);
+  }
+  k_edge_out<<<1, 1024, 0, es>>>(c->v, c->dev, s.contrib, gated);
+  if (c->capturing) cudaEventRecord(c->join, c->side);
   k_apply_gather<<<g, b, 0, c->cs>>>(c->v, c->dev);
   const unsigned wb = walk_blocks(c->v.N2);
   k_apply_xchains_t<<<wb, 128, 0, c->cs>>>(c->v, c->dev);
   k_apply_xchains_w<<<wb, 128, 0, c->cs>>>(c->v, c->dev);
   k_apply_ychains_t<<<wb, 128, 0, c->cs>>>(c->v, c->dev);
   k_apply_ychains_w<<<wb, 128, 0, c->cs>>>(c->v, c->dev);
-  count_launch(c, 6);
-  k_edge_out<<<1, 1024, 0, c->cs>>>(c->v, c->dev, s.contrib, gated);
-  count_launch(c, 1);
+  if (c->capturing) cudaStreamWaitEvent(c->cs, c->join, 0);
+  count_launch(c, 7);
 }
 
 void launch_lateral_check(hc_ctx* c) {

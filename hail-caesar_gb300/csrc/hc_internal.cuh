@@ -230,6 +230,8 @@ struct hc_ctx {
                           // conditional node's body is captured)
   cudaStream_t s2;
   cudaStream_t s3;         // snapshots to host memory (hc_snapshot_begin)
+  cudaStream_t side;       // a second branch of a captured iteration, with
+  cudaEvent_t fork, join;  // the events that split and join it
   hc_iter_handles hcur;   // handles of the iteration being captured
   int device;
   char err[512];
