@@ -215,6 +215,7 @@ extern "C" void* hc_stream(hc_ctx* c) { return c ? (void*)c->s : nullptr; }
 
 // ------------------------------------------------------------------ create
 static hc_status free_all(hc_ctx* c);
+static void snapshot_free(hc_snapshot* sn);
 
 hc_divisor host_divisor(double b) {
   unsigned long long B;
@@ -407,6 +408,7 @@ static hc_status free_all(hc_ctx* c) {
   if (c->s) cudaStreamDestroy(c->s);
   if (c->s2) cudaStreamDestroy(c->s2);
   if (c->s3) cudaStreamDestroy(c->s3);
+  for (hc_snapshot* sn : c->snaps) snapshot_free(sn);
   if (c->side) cudaStreamDestroy(c->side);
   if (c->fork) cudaEventDestroy(c->fork);
   if (c->join) cudaEventDestroy(c->join);
@@ -661,11 +663,24 @@ extern "C" hc_status hc_download(hc_ctx* c, hc_field f, void* host, size_t nbyte
 // ------------------------------------------------------------------ snapshots
 // A field's copy taken in stream order (a device-to-device copy, so the run
 // can go on at once) and moved to pinned host memory on a side stream.
+// A context keeps the buffers and events of up to kSnapKeep ended snapshots
+// for its next ones (freed with it): allocating and freeing them per snapshot,
+// which waits for the device, took 120 us each (four steps member by member at
+// 900 x 1400 with three rasters: 1.48 -> 1.15 ms).
 struct hc_snapshot {
   hc_ctx* c;
   double* dev;
+  size_t bytes;
   cudaEvent_t taken, done;
 };
+
+static void snapshot_free(hc_snapshot* sn) {
+  if (!sn) return;
+  if (sn->taken) cudaEventDestroy(sn->taken);
+  if (sn->done) cudaEventDestroy(sn->done);
+  if (sn->dev) cudaFree(sn->dev);
+  delete sn;
+}
 
 extern "C" hc_status hc_snapshot_begin(hc_ctx* c, hc_field f, void* host_pinned, size_t nbytes,
                                        hc_snapshot** out) {
@@ -674,21 +689,38 @@ extern "C" hc_status hc_snapshot_begin(hc_ctx* c, hc_field f, void* host_pinned,
   double* src = plain_field(c, f);
   if (!src) return hc_fail(c, HC_ERR_ARG, "field %d has no plain layout for a snapshot", (int)f);
   HC_TRY(check_size(c, f, nbytes));
-  hc_snapshot* sn = new hc_snapshot();
-  sn->c = c;
-  if (cudaMalloc((void**)&sn->dev, nbytes) != cudaSuccess) {
-    cudaGetLastError();
-    delete sn;
-    return hc_fail(c, HC_ERR_NOMEM, "snapshot buffer");
+  hc_snapshot* sn = nullptr;
+  for (auto& k : c->snaps)
+    if (!sn && k && k->bytes >= nbytes) {
+      sn = k;
+      k = nullptr;
+    }
+  if (!sn) {
+    sn = new hc_snapshot();
+    sn->c = c;
+    sn->bytes = nbytes;
+    if (cudaMalloc((void**)&sn->dev, nbytes) != cudaSuccess) {
+      cudaGetLastError();
+      snapshot_free(sn);
+      return hc_fail(c, HC_ERR_NOMEM, "snapshot buffer");
+    }
+    cudaEventCreateWithFlags(&sn->taken, cudaEventDisableTiming);
+    cudaEventCreateWithFlags(&sn->done, cudaEventDisableTiming);
   }
-  cudaEventCreateWithFlags(&sn->taken, cudaEventDisableTiming);
-  cudaEventCreateWithFlags(&sn->done, cudaEventDisableTiming);
-  HC_CU(cudaMemcpyAsync(sn->dev, src, nbytes, cudaMemcpyDeviceToDevice, c->s), "snapshot");
-  if (!c->s3) HC_CU(cudaStreamCreateWithFlags(&c->s3, cudaStreamNonBlocking), "snapshot stream");
-  HC_CU(cudaEventRecord(sn->taken, c->s), "snapshot");
-  HC_CU(cudaStreamWaitEvent(c->s3, sn->taken, 0), "snapshot");
-  HC_CU(cudaMemcpyAsync(host_pinned, sn->dev, nbytes, cudaMemcpyDeviceToHost, c->s3), "snapshot");
-  HC_CU(cudaEventRecord(sn->done, c->s3), "snapshot");
+  hc_status st = hc_cuda(c, cudaMemcpyAsync(sn->dev, src, nbytes, cudaMemcpyDeviceToDevice, c->s),
+                         "snapshot");
+  if (st == HC_OK && !c->s3)
+    st = hc_cuda(c, cudaStreamCreateWithFlags(&c->s3, cudaStreamNonBlocking), "snapshot stream");
+  if (st == HC_OK) st = hc_cuda(c, cudaEventRecord(sn->taken, c->s), "snapshot");
+  if (st == HC_OK) st = hc_cuda(c, cudaStreamWaitEvent(c->s3, sn->taken, 0), "snapshot");
+  if (st == HC_OK)
+    st = hc_cuda(c, cudaMemcpyAsync(host_pinned, sn->dev, nbytes, cudaMemcpyDeviceToHost, c->s3),
+                 "snapshot");
+  if (st == HC_OK) st = hc_cuda(c, cudaEventRecord(sn->done, c->s3), "snapshot");
+  if (st != HC_OK) {
+    snapshot_free(sn);
+    return st;
+  }
   c->d2h_bytes += nbytes;
   *out = sn;
   return HC_OK;
@@ -698,10 +730,13 @@ extern "C" hc_status hc_snapshot_end(hc_snapshot* sn) {
   if (!sn) return HC_ERR_ARG;
   hc_ctx* c = sn->c;
   const cudaError_t e = cudaEventSynchronize(sn->done);
-  cudaEventDestroy(sn->taken);
-  cudaEventDestroy(sn->done);
-  cudaFree(sn->dev);
-  delete sn;
+  if (e == cudaSuccess)
+    for (auto& k : c->snaps)
+      if (!k) {
+        k = sn;
+        return HC_OK;
+      }
+  snapshot_free(sn);
   return hc_cuda(c, e, "snapshot");
 }
 

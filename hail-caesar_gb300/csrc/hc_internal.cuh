@@ -223,6 +223,10 @@ struct hc_iter_handles {
 
 constexpr int kMaxFlowShapes = 24;  // launch shapes of k_flow_route the tuner can time
 
+// ended snapshots a context keeps (a device copy of a field each): what an
+// output step of a run writes side by side
+constexpr int kSnapKeep = 4;
+
 struct hc_ctx {
   hc_view v;
   cudaStream_t s;         // the context's stream
@@ -230,6 +234,7 @@ struct hc_ctx {
                           // conditional node's body is captured)
   cudaStream_t s2;
   cudaStream_t s3;         // snapshots to host memory (hc_snapshot_begin)
+  struct hc_snapshot* snaps[kSnapKeep];  // ended snapshots whose buffers are used again
   cudaStream_t side;       // a second branch of a captured iteration, with
   cudaEvent_t fork, join;  // the events that split and join it
   hc_iter_handles hcur;   // handles of the iteration being captured
