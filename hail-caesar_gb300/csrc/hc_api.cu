@@ -299,6 +299,7 @@ extern "C" hc_status hc_create(const hc_params* p, size_t max_bytes, hc_ctx** ou
   A(v.edge, E2) A(v.edge2, E2) A(v.veg, 4 * E2)
   A(v.cin_x, (size_t)p->imax * p->jmax + 2) A(v.cin_y, (size_t)p->imax * p->jmax + 2)
   A(v.wet, N2) A(v.wet_sums, (N2 + 1023) / 1024 + 1)
+  A(v.wet_bits, (size_t)p->imax * ((p->jmax + 31) / 32))
   // partial sums: one per block of scan_area (32 x 8 cells) or of a grid_sum
   v.vpart_cap = (int)std::max<size_t>(
       (size_t)((p->jmax + 31) / 32) * (size_t)((p->imax + 7) / 8), 152 * 8);
@@ -394,7 +395,7 @@ static hc_status free_all(hc_ctx* c) {
                   v.edge, v.edge2, v.veg, v.cin_x, v.cin_y, v.erodetot, v.erodetot3, v.pre,
                   v.chains, v.ent_list, v.ent_qs, v.drain_pos, v.drain_f0, v.drain_f1, v.drain_pend, v.drain_dt, v.drain_share, v.drain_head,
                   v.drain_snap, v.drain_aux, v.alloc_key, v.red, v.touched, v.topm, v.rain, v.rec, c->dev, v.wet,
-                  v.wet_sums, v.vpart, v.flux, v.sdirty, v.border,
+                  v.wet_sums, v.wet_bits, v.vpart, v.flux, v.sdirty, v.border,
                   v.reach[0], v.reach[1], v.reach[2], extra(c).lateral};
   for (void* q : ptrs)
     if (q) cudaFree(q);

@@ -943,29 +943,75 @@ __global__ void __launch_bounds__(256, 6) k_depth_update(const hc_view c, hc_dev
 // ---------------------------------------------------------------------------
 // scan_area :3821-3849 (every scan_area_interval_iter iterations)
 // ---------------------------------------------------------------------------
+// A warp takes 32 columns of kScanRows rows: each row's wet cells as one
+// ballot (with a bit from either side), a cell is listed when its own bit or
+// one of the eight around it is set, so three rows' words combine to the
+// mask's word.  The words, 32 cells each, are what the list is counted and
+// written from.
 // Also the ledger's volume: the depth sum of its block (rows 1..imax,
-// columns 1..jmax) into vpart, added up in order by k_wet_count's last block.
+// columns 1..jmax) into vpart, added up in order by k_wet_count's last block;
+// a lane adds its rows first, which costs one FP64 instruction per 32 cells
+// where a tree per row cost five.  The scan and the list, a thread per cell
+// before: 503 -> 127 us at 4001 x 4103; with the launches of a step that is
+// not due, 50 -> 22 us an iteration at 2000^2.
+constexpr int kScanRows = 8;
+
+// words of 32 columns in a row of the mask (columns 1..jmax)
+__host__ __device__ __forceinline__ int mask_words(int jmax) { return (jmax + 31) / 32; }
+
 __global__ void __launch_bounds__(256) k_scan_area(const hc_view c, const hc_dev* __restrict__ d,
                                                     int gated) {
   if (gated && !(d->it_active && d->do_scan)) return;
-  const int j = 1 + blockIdx.x * blockDim.x + threadIdx.x;
-  const int i = 1 + blockIdx.y * blockDim.y + threadIdx.y;
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x, w = blockIdx.x, wpr = gridDim.x;
+  const int i0 = 1 + (blockIdx.y * blockDim.y + threadIdx.y) * kScanRows;
+  const size_t W = c.W;
+  const int j = 1 + 32 * w + lane;  // columns 0 and jmax+1 are padding, and neighbours
+  const int js = lane == 0 ? j - 1 : j + 1;
+  const bool in = j <= c.jmax + 1, side = (lane == 0 || lane == 31) && js <= c.jmax + 1;
   double v = 0;
-  if (i <= c.imax && j <= c.jmax) {
-    const size_t W = c.W;
-    const size_t cell = (size_t)i * W + j;
-    const double* h = c.h;
-    v = h[cell];
-    bool wet = v > 0 || h[cell - 1] > 0 || h[cell + 1] > 0 || h[cell - W] > 0 ||
-               h[cell - W - 1] > 0 || h[cell - W + 1] > 0 || h[cell + W - 1] > 0 ||
-               h[cell + W + 1] > 0 || h[cell + W] > 0;
-    c.mask[cell] = wet ? 1 : 0;
+  if (i0 <= c.imax) {
+    double h[kScanRows + 2], x[kScanRows + 2];
+#pragma unroll
+    for (int q = 0; q < kScanRows + 2; q++) {
+      const int i = i0 - 1 + q;
+      const bool row = i <= c.imax + 1;
+      h[q] = row && in ? c.h[(size_t)i * W + j] : 0.0;
+      x[q] = row && side ? c.h[(size_t)i * W + js] : 0.0;
+    }
+    const unsigned cols = c.jmax - 32 * w >= 32 ? FULL : (1u << (c.jmax - 32 * w)) - 1u;
+    unsigned m2 = 0, m1 = 0;  // the two rows before, each with its neighbours in the row
+#pragma unroll
+    for (int q = 0; q < kScanRows + 2; q++) {
+      const unsigned b = __ballot_sync(FULL, dpos(h[q])), e = __ballot_sync(FULL, dpos(x[q]));
+      const unsigned m0 = b | (b << 1) | (b >> 1) | (e & 0x80000001u);
+      const int i = i0 - 2 + q;  // the row between the three
+      if (q >= 2 && i <= c.imax) {
+        const unsigned wet = (m2 | m1 | m0) & cols;
+        if (j <= c.jmax) {
+          c.mask[(size_t)i * W + j] = (uint8_t)((wet >> lane) & 1u);
+          v += h[q - 1];
+        }
+        if (lane == 0) c.wet_bits[(size_t)(i - 1) * wpr + w] = wet;
+      }
+      m2 = m1;
+      m1 = m0;
+    }
   }
   const double bsum = block_sum(v);
   if (threadIdx.x == 0 && threadIdx.y == 0) c.vpart[blockIdx.x + blockIdx.y * gridDim.x] = bsum;
 }
 
-// The wet list: mask bytes counted per block of 1024 cells, the counts
+// the words of a mask that was uploaded
+__global__ void __launch_bounds__(256) k_mask_words(const hc_view c) {
+  const int w = blockIdx.x, i = 1 + blockIdx.y * blockDim.y + threadIdx.y;
+  const int j = 1 + 32 * w + threadIdx.x;
+  const bool on = i <= c.imax && j <= c.jmax && c.mask[(size_t)i * c.W + j];
+  const unsigned b = __ballot_sync(0xffffffffu, on);
+  if (threadIdx.x == 0 && i <= c.imax) c.wet_bits[(size_t)(i - 1) * gridDim.x + w] = b;
+}
+
+// The wet list: the mask's words counted per block of 1024, the counts
 // scanned, the cell numbers written in ascending order.
 // The block counts, then, in the block that finishes last, their exclusive
 // scan (the wet list's offsets per block) and the list's length.  nvol:
@@ -975,15 +1021,14 @@ __global__ void __launch_bounds__(1024) k_wet_count(const hc_view c, hc_dev* d, 
                                                     int nvol) {
   __shared__ int ws[32];
   if (gated && !(d->it_active && d->do_scan)) return;
+  const size_t n = (size_t)c.imax * mask_words(c.jmax);
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  int v = (i < c.N2) ? c.mask[i] : 0;
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  const int v = __reduce_add_sync(0xffffffffu, (i < n) ? __popc(c.wet_bits[i]) : 0);
   if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = v;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    int s = 0;
-    for (int k = 0; k < 32; k++) s += ws[k];
-    c.wet_sums[blockIdx.x] = s;
+  if (threadIdx.x < 32) {
+    const int s = __reduce_add_sync(0xffffffffu, ws[threadIdx.x]);
+    if (threadIdx.x == 0) c.wet_sums[blockIdx.x] = s;
   }
   if (!last_to_arrive(&d->wet_arrive)) return;
   if (nvol > 0) {
@@ -999,32 +1044,48 @@ __global__ void __launch_bounds__(1024) k_wet_count(const hc_view c, hc_dev* d, 
   if (threadIdx.x == 0) d->wet_count = total;
 }
 
+// A thread's word gives its place in the list and its border cells (those
+// with an unlisted one of the four neighbours); then each warp writes its 32
+// words' cells, a word at a time.
 __global__ void __launch_bounds__(1024) k_wet_write(const hc_view c, const hc_dev* d, int gated) {
-  __shared__ int ws[32], wb[32];
+  __shared__ int ws[32];
   if (gated && !(d->it_active && d->do_scan)) return;
+  const unsigned FULL = 0xffffffffu;
+  const int wpr = mask_words(c.jmax);
+  const size_t n = (size_t)c.imax * wpr;
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int v = (i < c.N2) ? c.mask[i] : 0;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int incl = v;
+  unsigned m = 0, border = 0;
+  int first = 0, cols = 0;  // the word's first cell, its columns
+  if (i < n) {
+    const int r = (int)((unsigned)i / (unsigned)wpr), w = (int)i - r * wpr;
+    m = c.wet_bits[i];
+    const unsigned up = r > 0 ? c.wet_bits[i - wpr] : 0u;
+    const unsigned down = r < c.imax - 1 ? c.wet_bits[i + wpr] : 0u;
+    const unsigned left = (m << 1) | (w > 0 ? c.wet_bits[i - 1] >> 31 : 0u);
+    const unsigned right = (m >> 1) | (w < wpr - 1 ? c.wet_bits[i + 1] << 31 : 0u);
+    border = m & ~(up & down & left & right);
+    first = (int)((size_t)(r + 1) * c.W) + 1 + 32 * w;
+    cols = min(32, c.jmax - 32 * w);
+  }
+  const int cnt = __popc(m);
+  int incl = cnt;
   for (int o = 1; o < 32; o <<= 1) {
-    const int t = __shfl_up_sync(0xffffffffu, incl, o);
+    const int t = __shfl_up_sync(FULL, incl, o);
     if (lane >= o) incl += t;
   }
   if (lane == 31) ws[warp] = incl;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    int s = 0;
-    for (int k = 0; k < 32; k++) {
-      wb[k] = s;
-      s += ws[k];
-    }
+  int place = c.wet_sums[blockIdx.x] + incl - cnt;
+#pragma unroll
+  for (int k = 0; k < 32; k++) place += k < warp ? ws[k] : 0;
+#pragma unroll 4
+  for (int k = 0; k < 32; k++) {
+    const unsigned mk = __shfl_sync(FULL, m, k), bk = __shfl_sync(FULL, border, k);
+    const int at = __shfl_sync(FULL, place, k), f = __shfl_sync(FULL, first, k);
+    if ((mk >> lane) & 1u) c.wet[at + __popc(mk & ((1u << lane) - 1u))] = f + lane;
+    if (lane < __shfl_sync(FULL, cols, k)) c.border[f + lane] = (uint8_t)((bk >> lane) & 1u);
   }
-  __syncthreads();
-  if (v) c.wet[c.wet_sums[blockIdx.x] + wb[warp] + incl - 1] = (int32_t)i;
-  // the wet list's border (listed cells are in rows 1..imax, columns
-  // 1..jmax, so their four neighbours lie inside the padded grid)
-  if (i < c.N2)
-    c.border[i] = v && !(c.mask[i - 1] && c.mask[i + 1] && c.mask[i - c.W] && c.mask[i + c.W]);
 }
 
 // ---------------------------------------------------------------------------
@@ -1311,16 +1372,23 @@ static void wet_list(hc_ctx* c, int gated, int nvol);
 
 void launch_scan_area(hc_ctx* c, int gated) {
   dim3 b(32, 8);
-  const dim3 g = grid2d(c, b);
+  const int rows = 8 * kScanRows;
+  const dim3 g(mask_words(c->v.jmax), (c->v.imax + rows - 1) / rows);
   k_scan_area<<<g, b, 0, c->cs>>>(c->v, c->dev, gated);
   count_launch(c, 1);
   wet_list(c, gated, (int)(g.x * g.y));
 }
 
-void launch_wet_list(hc_ctx* c, int gated) { wet_list(c, gated, 0); }
+void launch_wet_list(hc_ctx* c, int gated) {
+  const dim3 g(mask_words(c->v.jmax), (c->v.imax + 7) / 8);
+  k_mask_words<<<g, dim3(32, 8), 0, c->cs>>>(c->v);
+  count_launch(c, 1);
+  wet_list(c, gated, 0);
+}
 
 static void wet_list(hc_ctx* c, int gated, int nvol) {
-  const int nb = (int)((c->v.N2 + 1023) / 1024);
+  const size_t words = (size_t)c->v.imax * mask_words(c->v.jmax);
+  const int nb = (int)((words + 1023) / 1024);
   k_wet_count<<<nb, 1024, 0, c->cs>>>(c->v, c->dev, gated, nvol);
   k_wet_write<<<nb, 1024, 0, c->cs>>>(c->v, c->dev, gated);
   count_launch(c, 2);

@@ -157,6 +157,8 @@ struct hc_view {
   int32_t *wet;                // cells of the wet mask, ascending (the down_scan
                                // lists as one array); length in hc_dev::wet_count
   int32_t *wet_sums;           // per-block counts for building it
+  uint32_t *wet_bits;          // the mask as words of 32 columns, row by row, while the list
+                               // is built
   uint32_t *ent_list;          // cells with flow in an entrainment pass (N2)
   double *ent_qs;              // their qtot and slope sum (2 per entry)
   int cin_cap;
@@ -431,6 +433,10 @@ HC_DEV double imax_d(double a, double b) { return dlt(a, b) ? b : a; }
 // 0 - x (the reference's spelling of a negation: +0 for x = +0)
 HC_DEV double zero_minus(double x) {
   return deq0(x) ? 0.0 : bits_d(dbits(x) ^ (long long)0x8000000000000000ULL);
+}
+// x > 0, a NaN of either sign excluded
+HC_DEV bool dpos(double x) {
+  return (unsigned long long)(dbits(x) - 1) < 0x7ff0000000000000ULL;
 }
 // x is a NaN
 HC_DEV bool disnan(double x) {
