@@ -54,11 +54,11 @@ static __device__ __noinline__ double einstein_td(double mts, double einA, hc_di
 static __device__ __noinline__ double ddiv_rn_entrain(double a, double b) { return ddiv_rn(a, b); }
 
 // blocks of 128 threads of the transport kernel (grid-stride over its
-// list): 1216 on large grids, fewer on small ones, whose lists are short and
+// list): 1216 on large grids, one per 128 cells on small ones, whose lists are short and
 // whose idle blocks would only cost dispatch (ensembles of small members run
 // many such launches side by side)
 static unsigned entrain_blocks(size_t N2) {
-  return (unsigned)std::min<size_t>(152 * 8, std::max<size_t>(16, N2 / 1024));
+  return (unsigned)std::min<size_t>(152 * 8, std::max<size_t>(16, N2 / 128));
 }
 
 __global__ void k_erode_begin(const hc_view c, hc_dev* d, int gated, double mult_override) {
@@ -160,8 +160,53 @@ __global__ void __launch_bounds__(128) k_entrain_tau(const hc_view c, hc_dev* d)
   }
 }
 
+// The transport of one fraction n of a cell (:4390-4440) before the bedrock
+// test: the amount that leaves, capped by what the record holds and, for the
+// suspended fraction, by the water's capacity.
+struct EntrainCell {
+  double h, tau, mts, Fs, d_50, graintot;  // the last three: Wilcock
+  hc_divisor Bd;                           // tau/g (Einstein)
+};
+
+__device__ __forceinline__ double entrain_fraction(const hc_view& c, size_t cell, int n,
+                                                   const EntrainCell& q) {
+  const hc_params& p = c.p;
+  const double rho = 1000.0, tau = q.tau, d_50 = q.d_50;
+  const double Di = p.d[n];
+  double td = 0;
+  if (p.wilcock) {
+    double tau_ri = (0.021 + (0.015 * exp(-20 * q.Fs))) * (rho * kG * d_50) *
+                    pow((Di / d_50), (0.67 / (1 + exp(1.5 - (Di / d_50)))));
+    // pow(tau / rho, 0.5): the square root, correctly rounded
+    double U_star = isqrt_rn(tau / rho);
+    double Fi = GRN(c, cell, n) / q.graintot;
+    double Wi_star;
+    if ((tau / tau_ri) < 1.35)
+      Wi_star = 0.002 * pow(tau / tau_ri, 7.5);
+    else
+      Wi_star = 14 * pow(1 - (0.894 / sqrt(tau / tau_ri)), 4.5);
+    td = ddiv_by(q.mts * ((Fi * (U_star * U_star * U_star)) / ((2.65 - 1) * kG)) * Wi_star, c.dxd);
+  }
+  if (p.einstein) td = einstein_td(q.mts, c.einA[n], q.Bd, c.einSd[n], c.dxd);
+  const double held = GRN(c, cell, n);
+  if (dgt(td, held)) td = held;
+  if (p.isSuspended[n] && n == 1) {
+    if (dgt(ddiv_rn_entrain(td + c.vs[cell], q.h), p.Csuspmax)) td = (q.h * p.Csuspmax) - c.vs[cell];
+  }
+  if (dlt0(td)) td = 0;
+  return td;
+}
+
 // The shear stress (:4316-4333) and the transport (:4388-4548) of one
 // listed cell (qtot > 0); returns temptot1.
+//
+// kHalf false: one thread per cell, the fractions in turn.  kHalf true: 16
+// lanes per cell, lane n with fraction n, for lists too short to fill the
+// GPU with a thread per cell: what a pass takes then is one cell's latency,
+// nine transports one after the other (Wilcock: three exponentials and powers
+// each) or one.  Sums over the fractions run over the lanes in the same order,
+// so the results are the same.
+template <bool kHalf>
 __device__ double entrain_cell(const hc_view& c, hc_dev* d, size_t cell, double mult,
                                double ts, double qtot, double slopetot) {
   const hc_params& p = c.p;
@@ -169,19 +214,21 @@ __device__ double entrain_cell(const hc_view& c, hc_dev* d, size_t cell, double 
   const int ix = (int)(cell / W), jy = (int)(cell % W);
   const double thr = p.water_depth_erosion_threshold;
   const double h = c.h[cell];
+  const int mine = kHalf ? (int)(threadIdx.x & 15) : 0;  // the lane's fraction
+  const unsigned half = kHalf ? 0xffffu << (threadIdx.x & 16) : 0u;
+  const bool lead = mine == 0;  // stores what the cell has one of
   double tau;
   {
     double vel = isqrt_rn(qtot);
-    c.vel[cell] = vel;
+    if (lead) c.vel[cell] = vel;
     if (dgt(vel, p.max_vel)) vel = p.max_vel;
     const double n_man = p.spatially_var_mannings ? c.man[cell] : p.mannings;
     const double ci = kG * (n_man * n_man) * pow(h, -0.33);
     if (dgt0(slopetot)) slopetot = 0;
     tau = 1000 * ci * vel * vel * (1 + (1 * ddiv_rn(slopetot, vel)));
-    c.tau[cell] = tau;
+    if (lead) c.tau[cell] = tau;
     if (!dgt0(tau)) return 0;  // no transport from this cell
   }
-  const double rho = 1000.0;
   const double e0 = c.elev[cell];
   const unsigned long long pos = (unsigned long long)jy * (c.imax + 2) + ix;
   // the direction weights of the velocity pass (:4250-4289), again
@@ -204,76 +251,72 @@ __device__ double entrain_cell(const hc_view& c, hc_dev* d, size_t cell, double 
       }
     }
   }
-  double temp_dist[HC_G] = {0};
-  double d_50 = 0, Fs = 0, graintot = 0;
+  EntrainCell q;
+  q.h = h;
+  q.tau = tau;
+  q.mts = mult * ts;
+  q.d_50 = q.Fs = q.graintot = 0;
   if (p.wilcock) {
-    d_50 = d50_dev(c, cell);
-    if (d_50 < p.d[1]) d_50 = p.d[1];
-    Fs = sand_fraction_dev(c, cell);
-    for (int n = 1; n <= HC_G; n++) graintot += GRN(c, cell, n);
+    q.d_50 = d50_dev(c, cell);
+    if (q.d_50 < p.d[1]) q.d_50 = p.d[1];
+    q.Fs = sand_fraction_dev(c, cell);
+    for (int n = 1; n <= HC_G; n++) q.graintot += GRN(c, cell, n);
   }
-  double temptot1 = 0;
-  const double mts = mult * ts;
   // Einstein: 1 / ((1650 Di) / (tau/g)); the nine quotients by tau/g
   // share one prepared divisor
-  const double Bq = ddiv_rn(tau, kG);
-  const hc_divisor Bd = ddiv_prep(Bq);
-  for (int n = 1; n <= HC_G - 1; n++) {
-    const double Di = p.d[n];
-    double td = 0;
-    if (p.wilcock) {
-      double tau_ri = (0.021 + (0.015 * exp(-20 * Fs))) * (rho * kG * d_50) *
-                      pow((Di / d_50), (0.67 / (1 + exp(1.5 - (Di / d_50)))));
-      // pow(tau / rho, 0.5): the square root, correctly rounded
-      double U_star = isqrt_rn(tau / rho);
-      double Fi = GRN(c, cell, n) / graintot;
-      double Wi_star;
-      if ((tau / tau_ri) < 1.35)
-        Wi_star = 0.002 * pow(tau / tau_ri, 7.5);
-      else
-        Wi_star = 14 * pow(1 - (0.894 / sqrt(tau / tau_ri)), 4.5);
-      td = ddiv_by(mts * ((Fi * (U_star * U_star * U_star)) / ((2.65 - 1) * kG)) * Wi_star,
-                   c.dxd);
+  q.Bd = ddiv_prep(ddiv_rn(tau, kG));
+  double temp_dist[HC_G] = {0};  // kHalf: [0] is the lane's
+  double temptot1 = 0;
+  auto sum_lanes = [&](double v) {
+    double t = 0;
+    for (int n = 1; n <= HC_G - 1; n++) t += __shfl_sync(half, v, n, 16);
+    return t;
+  };
+  if (kHalf) {
+    if (mine >= 1 && mine <= HC_G - 1) temp_dist[0] = entrain_fraction(c, cell, mine, q);
+    temptot1 = sum_lanes(temp_dist[0]);
+  } else {
+    for (int n = 1; n <= HC_G - 1; n++) {
+      temp_dist[n] = entrain_fraction(c, cell, n, q);
+      temptot1 += temp_dist[n];
     }
-    if (p.einstein) td = einstein_td(mts, c.einA[n], Bd, c.einSd[n], c.dxd);
-    if (dgt(td, GRN(c, cell, n))) td = GRN(c, cell, n);
-    if (p.isSuspended[n] && n == 1) {
-      if (dgt((td + c.vs[cell]) / h, p.Csuspmax)) td = (h * p.Csuspmax) - c.vs[cell];
-    }
-    if (dlt0(td)) td = 0;
-    temp_dist[n] = td;
-    temptot1 += td;
   }
   const double bed = c.bed[cell];
   if (!dgt(e0 - temptot1, bed)) {
     double elevdiff = e0 - bed;
     double temptot3 = temptot1;
-    temptot1 = 0;
-    for (int n = 1; n <= HC_G - 1; n++) {
-      if (!dgt(e0, bed)) {
-        temp_dist[n] = 0;
-      } else {
-        temp_dist[n] = elevdiff * ddiv_rn_entrain(temp_dist[n], temptot3);
-        if (dlt0(temp_dist[n])) temp_dist[n] = 0;
+    auto rescaled = [&](double t) {
+      if (!dgt(e0, bed)) return 0.0;
+      t = elevdiff * ddiv_rn_entrain(t, temptot3);
+      return dlt0(t) ? 0.0 : t;
+    };
+    if (kHalf) {
+      if (mine >= 1 && mine <= HC_G - 1) temp_dist[0] = rescaled(temp_dist[0]);
+      temptot1 = sum_lanes(temp_dist[0]);
+    } else {
+      temptot1 = 0;
+      for (int n = 1; n <= HC_G - 1; n++) {
+        temp_dist[n] = rescaled(temp_dist[n]);
+        temptot1 += temp_dist[n];
       }
-      temptot1 += temp_dist[n];
     }
     if (dgt(tau, p.bedrock_erosion_threshold)) {
       double amount = pow(p.bedrock_erosion_rate * tau, 1.5) * ts * mult * 0.000000317;
-      c.bed[cell] = bed - amount;
-      for (int n2 = 1; n2 <= HC_G - 1; n2++) GRN(c, cell, n2) += amount * p.dprop[n2];
+      if (lead) c.bed[cell] = bed - amount;
+      for (int n2 = 1; n2 <= HC_G - 1; n2++)
+        if (!kHalf || n2 == mine) GRN(c, cell, n2) += amount * p.dprop[n2];
     }
   }
   // vegetation terms (:4459-4488) vanish: vegetation is not supported
   // (hc_create rejects vegetation_on) and veg stays zero.
   if (dgt0(temptot1)) {
-    c.sdirty[cell] = 1;  // the next pass clears this cell's flux entries
+    if (lead) c.sdirty[cell] = 1;  // the next pass clears this cell's flux entries
     for (int k = 0; k < 4; k++) {
       const int pp = 1 + 2 * k;
       const int x2 = ix + kDXc[pp], y2 = jy + kDYc[pp];
       const size_t nb = (size_t)x2 * W + y2;
       if (dgt(c.h[nb], thr)) {
-        if (c.index[nb] < 1) {  // no final row number yet: ask
+        if (lead && c.index[nb] < 1) {  // no final row number yet: ask
           atomicMin(&c.alloc_key[nb], pos * 5 + 1 + k);
           d->alloc_count = 1;
         }
@@ -281,14 +324,15 @@ __device__ double entrain_cell(const hc_view& c, hc_dev* d, size_t cell, double 
         if (dgt0(c.vd[(size_t)k * N2 + cell])) factor += ddiv_rn(0.75 * tempdir[k], veltot);
         const double edge2 = c.edge[EX(c, x2, y2)];
         if (dgt(edge0, edge2)) factor += 0.25 * ddiv_rn(edge0 - edge2, temptot2);
-        for (int n = 1; n <= HC_G - 1; n++) {
-          if (dgt0(temp_dist[n])) {
-            if (n == 1 && p.isSuspended[n]) {
-              c.ss[cell] = temp_dist[n];
-            } else {
-              SF(c, k, n, cell) = temp_dist[n] * factor;
-            }
-          }
+        auto give = [&](int n, double t) {
+          if (!dgt0(t)) return;
+          if (n == 1 && p.isSuspended[n]) c.ss[cell] = t;
+          else SF(c, k, n, cell) = t * factor;
+        };
+        if (kHalf) {
+          if (mine >= 1 && mine <= HC_G - 1) give(mine, temp_dist[0]);
+        } else {
+          for (int n = 1; n <= HC_G - 1; n++) give(n, temp_dist[n]);
         }
       }
     }
@@ -305,10 +349,20 @@ __global__ void __launch_bounds__(128) k_entrain(const hc_view c, hc_dev* d, int
   const double mult = d->mult, ts = d->s.time_step;
   const unsigned n_list = *(volatile unsigned*)&d->ent_n;
   double tb = 0;
-  for (unsigned k = blockIdx.x * blockDim.x + threadIdx.x; k < n_list;
-       k += gridDim.x * blockDim.x)
-    tb = smax(tb, entrain_cell(c, d, c.ent_list[k], mult, ts, c.ent_qs[2 * (size_t)k],
-                               c.ent_qs[2 * (size_t)k + 1]));
+  // 16 lanes per cell while that takes the launch at most two turns of its
+  // threads.  An iteration of the 300 x 100 reach (3,000 cells listed, Wilcock):
+  // 261 -> 240 us, of 128 x 128 (Einstein) 136 -> 126.  Longer lists fill the GPU
+  // with a thread per cell, whose common terms are formed once, not 16 times.
+  const unsigned threads = gridDim.x * blockDim.x;
+  if (n_list <= threads / 8) {
+    for (unsigned k = (blockIdx.x * blockDim.x + threadIdx.x) >> 4; k < n_list; k += threads >> 4)
+      tb = smax(tb, entrain_cell<true>(c, d, c.ent_list[k], mult, ts, c.ent_qs[2 * (size_t)k],
+                                       c.ent_qs[2 * (size_t)k + 1]));
+  } else {
+    for (unsigned k = blockIdx.x * blockDim.x + threadIdx.x; k < n_list; k += threads)
+      tb = smax(tb, entrain_cell<false>(c, d, c.ent_list[k], mult, ts, c.ent_qs[2 * (size_t)k],
+                                        c.ent_qs[2 * (size_t)k + 1]));
+  }
   // tempbmax: max over the pass (warp shuffle, block, grid via last block)
   for (int o = 16; o > 0; o >>= 1) tb = smax(tb, __shfl_xor_sync(0xffffffffu, tb, o));
   const int t = threadIdx.x;
