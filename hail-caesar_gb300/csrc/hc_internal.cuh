@@ -209,8 +209,8 @@ struct hc_view {
   hc_step_record *rec; int64_t rec_cap;
   // test hook of the bounded device waits (hc_test_bounded_waits): when
   // wait_spins > 0 the drainage sweep's waits give up after that many spins,
-  // and its grid barrier expects barrier_extra arrivals more than there are
-  // blocks (with no single-block frontiers), so that every wait runs out
+  // and it expects barrier_extra cells more than there are, so that they run
+  // out
   int wait_spins, barrier_extra;
 };
 
