@@ -1026,34 +1026,12 @@ __global__ void __launch_bounds__(128) k_apply_ychains_t(const hc_view c, hc_dev
 // results are the serial loop's.  Rows r-1, r, r+1 are held (U, C, D) and
 // row r+2 is loaded while row r is worked on.
 // ---------------------------------------------------------------------------
-constexpr unsigned kFull = 0xffffffffu;
-
-struct WRow {
-  double g;  // grain plane `lane` (lanes 0..HC_G; 0 in the others)
-  double elev, h, bed, edge;
-  int idx;
-  bool dirty;
-};
-
 // the rest of a row the x walker needs when it is the current row
 struct WExtra {
   double pre;  // PRE plane `lane` (lanes 0..HC_G)
   double tau, ss, et3;
   bool mask;
 };
-
-__device__ __forceinline__ int lane_id() { return (int)(threadIdx.x & 31); }
-
-__device__ __forceinline__ void wrow_load(const hc_view& c, size_t cell, size_t ecell, WRow& r) {
-  const int L = lane_id();
-  r.g = (L <= HC_G) ? GRN(c, cell, L) : 0.0;
-  r.elev = c.elev[cell];
-  r.h = c.h[cell];
-  r.bed = c.bed[cell];
-  r.edge = c.edge[ecell];
-  r.idx = c.index[cell];
-  r.dirty = false;
-}
 
 __device__ __forceinline__ void wextra_load(const hc_view& c, size_t cell, bool with_pre,
                                             WExtra& x) {
@@ -1063,112 +1041,6 @@ __device__ __forceinline__ void wextra_load(const hc_view& c, size_t cell, bool 
   x.ss = c.ss[cell];
   x.et3 = c.erodetot3[cell];
   x.mask = c.mask[cell] != 0;
-}
-
-__device__ __forceinline__ void wrow_store(const hc_view& c, size_t cell, const WRow& r) {
-  if (!r.dirty) return;
-  const int L = lane_id();
-  if (L >= 1 && L <= HC_G - 1) GRN(c, cell, L) = r.g;
-  if (L == 0) c.elev[cell] = r.elev;
-}
-
-// sort_active on a held row, the warp together (same decisions as
-// sort_active_row; the float estimate's sum order does not matter, its
-// error bound holds for any order)
-__device__ void sort_active_w(const hc_view& c, hc_dev* d, size_t cell, WRow& r) {
-  const int L = lane_id();
-  if (r.idx == -9999) {
-    if (L == 0) {
-      d->err_code = 201;
-      d->pause |= HC_PAUSE_ERROR;
-    }
-    return;
-  }
-  const double active = c.p.active;
-  const float f = (L <= HC_G) ? approx_f(r.g) : 0.0f;
-  float sf = f, af = fabsf(f);
-  for (int o = 16; o > 0; o >>= 1) {
-    sf += __shfl_xor_sync(kFull, sf, o);
-    af += __shfl_xor_sync(kFull, af, o);
-  }
-  const float tol = 1e-5f * af + 1e-30f;
-  const float hi = c.act_hi, lo = c.act_lo;
-  const int dep = (sf > hi + tol) ? 1 : ((sf < hi - tol) ? -1 : 0);
-  const int ero = (sf < lo - tol) ? 1 : ((sf > lo + tol) ? -1 : 0);
-  if (dep == -1 && ero == -1) return;
-  double total = 0.0;  // in the reference's order, n = 0 .. HC_G
-  for (int n = 0; n <= HC_G; n++) total += __shfl_sync(kFull, r.g, n);
-  if (total > (active * 1.5)) {
-    if (L <= HC_G - 2)
-      for (int z = 9; z >= 1; z--) STR(c, cell, z, L) = STR(c, cell, z - 1, L);
-    __syncwarp();
-    const double coeff = active / total;
-    if (L >= 1 && L <= HC_G - 1 && r.g > 0.0) {
-      const double amount = coeff * (r.g);
-      STR(c, cell, 0, L - 1) = amount;
-      r.g = r.g - amount;
-    }
-    r.dirty = true;
-    __syncwarp();
-  }
-  if (total < (active / 4)) {
-    double s0 = 0;
-    if (L >= 1 && L <= HC_G - 1) s0 = STR(c, cell, 0, L - 1);
-    __syncwarp();
-    if (L <= HC_G - 2)
-      for (int z = 0; z <= 8; z++) STR(c, cell, z, L) = STR(c, cell, z + 1, L);
-    __syncwarp();
-    if (L >= 1 && L <= HC_G - 1) {
-      r.g += s0;
-      STR(c, cell, 9, L - 1) = active * c.p.dprop[L];
-    }
-    r.dirty = true;
-    __syncwarp();
-  }
-}
-
-// slide_GS(a -> b, amount) on held rows, the warp together
-__device__ void slide_GS_w(const hc_view& c, hc_dev* d, size_t a, WRow& A, double amount,
-                           size_t b, WRow& B) {
-  const int L = lane_id();
-  const bool fr = L >= 1 && L <= HC_G - 1;
-  const double dp = fr ? c.p.dprop[L] : 0.0;
-  const bool ha = A.idx != -9999, hb = B.idx != -9999;
-  if (ha && hb) {
-    double total = 0;  // positive fractions 1..9, in order
-    for (int n = 1; n <= HC_G - 1; n++) {
-      const double v = __shfl_sync(kFull, A.g, n);
-      if (dgt0(v)) total += v;
-    }
-    if (dgt(amount, total)) {
-      if (fr) B.g += (amount - total) * dp;
-      amount = total;
-    }
-    if (dgt0(total)) {
-      if (fr) {
-        const double ga = A.g;
-        const double t = amount * ddiv_rn(ga, total);
-        B.g += t;
-        double na = ga - t;
-        if (dlt0(na)) na = 0;
-        A.g = na;
-      }
-    }
-    A.dirty = B.dirty = true;
-    sort_active_w(c, d, a, A);
-    sort_active_w(c, d, b, B);
-    return;
-  }
-  if (!ha && hb) {
-    if (fr) B.g += (amount)*dp;
-    B.dirty = true;
-    sort_active_w(c, d, b, B);
-    return;
-  }
-  if (ha && !hb && L == 0) {
-    d->err_code = 202;
-    d->pause |= HC_PAUSE_ERROR;
-  }
 }
 
 __device__ __forceinline__ bool lateral_amount_w(const hc_params& p, const hc_divisor& dxd,

@@ -117,59 +117,66 @@ __device__ bool slide_probe_cell(const hc_view& c, int x, int y, double factor) 
   return false;
 }
 
-// slide_GS for a move of the replay.  When both records exist, on the
-// records held in registers (all loads issued together: the serial replay
-// waits on latency); out of line, so that the eight tests of a visit share
-// one copy of it.
-static __device__ __noinline__ void replay_slide_GS(const hc_view& c, hc_dev* d, size_t cell,
-                                                    double diff, size_t nb) {
-  if (c.index[cell] != -9999 && c.index[nb] != -9999) {
-    ApplyRow A, B;
-    row_load(c, cell, 0, A);
-    row_load(c, nb, 0, B);
-    slide_GS_rows(c, d, cell, A, diff, nb, B, positive_total(A));
-    row_store(c, cell, A);
-    row_store(c, nb, B);
-  } else {
-    slide_GS_dev(c, d, cell, diff, nb, true);
-  }
-}
+// Neighbour k of a visit, in the reference's order of tests (:5457-5522).
+__device__ __forceinline__ int nb_dx(int k) { return ((0xa406 >> (2 * k)) & 3) - 1; }
+__device__ __forceinline__ int nb_dy(int k) { return ((0x406a >> (2 * k)) & 3) - 1; }
 
-// The visit as the serial replay makes it (:5445-5525): the eight
-// neighbours' elevations are loaded together (one round trip instead of
-// eight dependent ones), each test is first decided on estimates
-// (drop_above_est) and formed in FP64 only when it may pass, and moves update
-// the held values.  The tests, moves and their order are the reference's;
-// returns the moved directions (bit k: neighbour k).
-__device__ int slide_visit_held(const hc_view& c, hc_dev* d, int x, int y, double factor) {
-  constexpr int dxs[8] = {1, 0, -1, -1, -1, 0, 1, 1};
-  constexpr int dys[8] = {1, 1, 1, 0, -1, -1, -1, 0};
+// The visit as the serial replay makes it (:5445-5525), by the warp: lane k
+// holds neighbour k's elevation and tests it (drop_above_est first, FP64 only
+// when it may pass) against the cell's elevation as the moves so far left it;
+// the first direction that passes moves, and the later ones are tested again.
+// Each test so sees the elevations the serial visit's would.  A move's grain
+// transfer runs with a fraction per lane (slide_GS_w): what it waits for is a
+// chain of FP64 operations, nine fractions one after the other in one thread.
+// By one thread, with its 35 mask bytes and 25 pushes in turn (now a lane
+// each, push_affected): slide_3 415 -> 288 us an iteration late in a storm at
+// 2000^2, 77 -> 68 us earlier in it.
+// Returns the moved directions (bit k: neighbour k).
+__device__ int slide_visit_warp(const hc_view& c, hc_dev* d, int x, int y, double factor) {
+  const int lane = lane_id(), k = lane & 7;
+  const bool diag = nb_dx(k) != 0 && nb_dy(k) != 0;
   const size_t W = c.W;
   const size_t cell = (size_t)x * W + y;
-  double en[8];
-#pragma unroll
-  for (int k = 0; k < 8; k++) en[k] = c.elev[(size_t)(x + dxs[k]) * W + (y + dys[k])];
+  const size_t nbc = (size_t)(x + nb_dx(k)) * W + (y + nb_dy(k));
+  const double e2 = c.elev[nbc];
   double e = c.elev[cell];
   const double floor_e = c.bed[cell] + c.p.active;
   const double wet_factor = (e <= floor_e) ? 10000.0 : factor;
-  const float fw = approx_f(wet_factor);
+  const float fe2 = approx_f(e2), fw = approx_f(wet_factor);
   int moved = 0;
-#pragma unroll
-  for (int k = 0; k < 8; k++) {
-    const bool diag = dxs[k] != 0 && dys[k] != 0;
-    const double e2 = en[k];
-    if (drop_above_est(approx_f(e), approx_f(e2), fw, diag) == 0) continue;
-    const double drop = diag ? ((e - e2) / 1.41) : (e - e2);
-    if (!(drop > wet_factor && e2 > -9999)) continue;
-    double diff = drop - wet_factor;
+  for (int from = 0; from < 8;) {
+    bool pass = false;
+    double drop = 0;
+    if (lane >= from && lane < 8 && drop_above_est(approx_f(e), fe2, fw, diag) != 0) {
+      drop = diag ? ((e - e2) / 1.41) : (e - e2);
+      pass = drop > wet_factor && e2 > -9999;
+    }
+    const unsigned ball = __ballot_sync(kFull, pass);
+    if (!ball) break;
+    const int m = __ffs(ball) - 1;
+    double diff = __shfl_sync(kFull, drop, m) - wet_factor;
     if ((e - diff) < floor_e) diff = (e - floor_e);
-    const size_t nb = (size_t)(x + dxs[k]) * W + (y + dys[k]);
+    const size_t nb = __shfl_sync(kFull, (unsigned long long)nbc, m);
     e = e - diff;
-    en[k] = e2 + diff;
-    c.elev[cell] = e;
-    c.elev[nb] = en[k];
-    replay_slide_GS(c, d, cell, diff, nb);
-    moved |= 1 << k;
+    const double en = __shfl_sync(kFull, e2, m) + diff;
+    if (lane == 0) {
+      c.elev[cell] = e;
+      c.elev[nb] = en;
+    }
+    __syncwarp();
+    WRow A, B;
+    wrow_load(c, cell, 0, A);
+    wrow_load(c, nb, 0, B);
+    if (A.idx != -9999 && B.idx != -9999) {
+      slide_GS_w(c, d, cell, A, diff, nb, B);
+      wrow_store(c, cell, A);
+      wrow_store(c, nb, B);
+    } else if (lane == 0) {
+      slide_GS_dev(c, d, cell, diff, nb, true);
+    }
+    __syncwarp();
+    moved |= 1 << m;
+    from = m + 1;
   }
   return moved;
 }
@@ -251,64 +258,49 @@ __global__ void k_flag_compact(const uint8_t* flag, size_t n, const int32_t* blo
 // The down_scan entries that visit row xx of column yy are xx itself and
 // the clamped entries 1 -> 2 and imax -> imax-1.  Returns the number of
 // positions newly set in the ring.
+//
+// By the warp: lane b holds cell b of the 5x5 block around (x, y).
 __device__ int push_affected(const hc_view& c, const Order& o, int x, int y, int moved, int Pcur,
                              uint32_t* ring, int RW) {
-  constexpr int dxs[8] = {1, 0, -1, -1, -1, 0, 1, 1};
-  constexpr int dys[8] = {1, 1, 1, 0, -1, -1, -1, 0};
-  // cells of the 5x5 block around (x, y) within one of a changed cell:
-  // bit (dx+2)*5 + (dy+2)
-  unsigned need = 0;
-#pragma unroll
-  for (int k = -1; k < 8; k++) {
-    if (k >= 0 && !((moved >> k) & 1)) continue;
-    const int cx = (k < 0) ? 0 : dxs[k], cy = (k < 0) ? 0 : dys[k];
-#pragma unroll
-    for (int dx = -1; dx <= 1; dx++)
-#pragma unroll
-      for (int dy = -1; dy <= 1; dy++) need |= 1u << ((cx + dx + 2) * 5 + (cy + dy + 2));
+  const int b = lane_id();
+  // cells within one of a changed cell: bit (dx+2)*5 + (dy+2)
+  constexpr unsigned kAround = 0x7u | 0x7u << 5 | 0x7u << 10;
+  unsigned need = kAround << 6;
+  for (int left = moved; left; left &= left - 1) {
+    const int k = __ffs(left) - 1;
+    need |= kAround << (6 + nb_dx(k) * 5 + nb_dy(k));
   }
-  // x and y lie in [2, imax-1] x [2, jmax-1], so every byte below is inside
-  // the padded grid: all 35 are loaded together, before any test
+  const int xx = x + b / 5 - 2, yy = y + b % 5 - 2;
+  const bool mine = b < 25 && ((need >> b) & 1u) && xx >= 2 && xx <= c.imax - 1 && yy >= 2 &&
+                    yy <= c.jmax - 1;
   const size_t W = c.W;
-  uint8_t mk[25], mt[5], mb[5];
-#pragma unroll
-  for (int b = 0; b < 25; b++) mk[b] = c.mask[(size_t)(x + b / 5 - 2) * W + (y + b % 5 - 2)];
-#pragma unroll
-  for (int j = 0; j < 5; j++) {
-    mt[j] = c.mask[W + (y + j - 2)];
-    mb[j] = c.mask[(size_t)c.imax * W + (y + j - 2)];
+  bool m0 = false, mt = false, mb = false;
+  if (mine) {
+    m0 = c.mask[(size_t)xx * W + yy];
+    mt = xx == 2 && c.mask[W + yy];
+    mb = xx == c.imax - 1 && c.mask[(size_t)c.imax * W + yy];
   }
-  int added = 0;
-  auto push = [&](int P) {
-    if (P <= Pcur) return;
-    uint32_t& w = ring[(P >> 5) & (RW - 1)];
-    const uint32_t bit = 1u << (P & 31);
-    if (!(w & bit)) {
-      w |= bit;
-      added++;
+  auto push = [&](bool want, int row) {
+    bool fresh = false;
+    if (want) {
+      const int P = o.pos(row, yy);
+      const uint32_t bit = 1u << (P & 31);
+      fresh = P > Pcur && !(atomicOr(&ring[(P >> 5) & (RW - 1)], bit) & bit);
     }
+    return __popc(__ballot_sync(kFull, fresh));
   };
-#pragma unroll
-  for (int b = 0; b < 25; b++) {
-    const int xx = x + b / 5 - 2, yy = y + b % 5 - 2;
-    if (!((need >> b) & 1u) || xx < 2 || xx > c.imax - 1 || yy < 2 || yy > c.jmax - 1) continue;
-    if (mk[b]) push(o.pos(xx, yy));
-    if (xx == 2 && mt[b % 5]) push(o.pos(1, yy));
-    if (xx == c.imax - 1 && mb[b % 5]) push(o.pos(c.imax, yy));
-  }
-  return added;
+  return push(m0, xx) + push(mt, 1) + push(mb, c.imax);
 }
 
 // The serial sweep in loop order over the flagged positions and the queued
 // re-tests, by one warp.  A visit that moves nothing changes nothing, so the
 // next kReplayBatch candidates in loop order are probed together, one per
 // lane, against the current elevations; the candidates before the first one
-// that moves are done, that one is visited in full by lane 0 (its moves
+// that moves are done, that one is visited in full (its moves
 // depend on the moves before it), and the candidates after it stay queued,
 // to be probed again on the changed elevations.  The visits and moves are
 // the serial sweep's, in its order.
 constexpr int kReplayBatch = 8;
-constexpr unsigned kFull = 0xffffffffu;
 
 __device__ __forceinline__ void replay_cell(const hc_view& c, const Order& o, int P, int& x,
                                             int& y) {
@@ -392,16 +384,12 @@ __global__ void __launch_bounds__(32) k_slide_replay(const hc_view c, hc_dev* d,
     if (tookL && upto == nb - 1) li++;
     last = batch[upto];
     if (ball) {
-      int added = 0;
-      if (lane == 0) {
-        int x, y;
-        replay_cell(c, o, last, x, y);
-        const int moved = slide_visit_held(c, d, x, y, factor);
-        if (moved) added = push_affected(c, o, x, y, moved, last, ring, RW);
-      }
-      pend += __shfl_sync(kFull, added, 0);
+      int x, y;
+      replay_cell(c, o, last, x, y);
+      const int moved = slide_visit_warp(c, d, x, y, factor);
+      if (moved) pend += push_affected(c, o, x, y, moved, last, ring, RW);
     }
-    // lane 0's moves and pushes are visible to the warp's next turn
+    // the moves and pushes are visible to the warp's next turn
     __syncwarp();
   }
   if (lane == 0) d->s.grain_array_tot = d->grain_tot;
