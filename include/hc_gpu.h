@@ -384,13 +384,13 @@ hc_status hc_get_run_stats(hc_ctx* ctx, int64_t* counts, double* host_ms, int32_
 
 /* Test hook of the bounded device waits (no counterpart in the reference).
  * The drainage recomputation (drainage_area_D8 :2091-2271) runs as one
- * cooperative kernel whose blocks wait for one another at grid barriers;
+ * kernel whose warps wait for cells that others release;
  * every such wait gives up after a bounded number of spins, and the call
  * that launched it returns HC_ERR_TIMEOUT with the context still usable (hc_run
  * then redoes the recomputation first thing in its next call).  spins > 0
- * sets that bound (0 restores the built-in ones) and makes each barrier
- * expect extra_arrivals more blocks than were launched, so that every wait
- * runs out: the way the tests check this path without a fault. */
+ * sets that bound (0 restores the built-in one) and makes the kernel expect
+ * extra_arrivals more cells than there are, so that the waits run out: the
+ * way the tests check this path without a fault. */
 hc_status hc_test_bounded_waits(hc_ctx* ctx, int32_t spins, int32_t extra_arrivals);
 
 /* Launch-shape autotuner (no counterpart in the reference).  hc_run times
