@@ -215,7 +215,7 @@ extern "C" void* hc_stream(hc_ctx* c) { return c ? (void*)c->s : nullptr; }
 
 // ------------------------------------------------------------------ create
 static hc_status free_all(hc_ctx* c);
-static void snapshot_free(hc_snapshot* sn);
+static void snapshots_detach(hc_ctx* c);
 
 hc_divisor host_divisor(double b) {
   unsigned long long B;
@@ -241,8 +241,9 @@ extern "C" hc_status hc_create(const hc_params* p, size_t max_bytes, hc_ctx** ou
     return HC_ERR_ARG;
   if (p->vegetation_on) return HC_ERR_UNSUPPORTED;
   if ((double)(p->imax + 2) * (p->jmax + 2) * 5 > 2147483647.0) return HC_ERR_UNSUPPORTED;
-  hc_ctx* c = new hc_ctx();
-  std::memset((void*)c, 0, sizeof *c);
+  hc_ctx* c = new hc_ctx();  // all zero
+  c->snaps = std::make_shared<hc_snap_pool>();
+  c->snaps->ctx = c;
   c->max_bytes = max_bytes;
   hc_view& v = c->v;
   v.p = *p;
@@ -409,7 +410,7 @@ static hc_status free_all(hc_ctx* c) {
   if (c->s) cudaStreamDestroy(c->s);
   if (c->s2) cudaStreamDestroy(c->s2);
   if (c->s3) cudaStreamDestroy(c->s3);
-  for (hc_snapshot* sn : c->snaps) snapshot_free(sn);
+  snapshots_detach(c);
   if (c->side) cudaStreamDestroy(c->side);
   if (c->fork) cudaEventDestroy(c->fork);
   if (c->join) cudaEventDestroy(c->join);
@@ -669,7 +670,7 @@ extern "C" hc_status hc_download(hc_ctx* c, hc_field f, void* host, size_t nbyte
 // which waits for the device, took 120 us each (four steps member by member at
 // 900 x 1400 with three rasters: 1.48 -> 1.15 ms).
 struct hc_snapshot {
-  hc_ctx* c;
+  std::shared_ptr<hc_snap_pool> pool;
   double* dev;
   size_t bytes;
   cudaEvent_t taken, done;
@@ -683,6 +684,16 @@ static void snapshot_free(hc_snapshot* sn) {
   delete sn;
 }
 
+// The context goes: its kept buffers are freed, its open snapshots live on.
+static void snapshots_detach(hc_ctx* c) {
+  std::lock_guard<std::mutex> lock(c->snaps->m);
+  c->snaps->ctx = nullptr;
+  for (auto& k : c->snaps->kept) {
+    snapshot_free(k);
+    k = nullptr;
+  }
+}
+
 extern "C" hc_status hc_snapshot_begin(hc_ctx* c, hc_field f, void* host_pinned, size_t nbytes,
                                        hc_snapshot** out) {
   if (!c || !host_pinned || !out) return HC_ERR_ARG;
@@ -691,14 +702,17 @@ extern "C" hc_status hc_snapshot_begin(hc_ctx* c, hc_field f, void* host_pinned,
   if (!src) return hc_fail(c, HC_ERR_ARG, "field %d has no plain layout for a snapshot", (int)f);
   HC_TRY(check_size(c, f, nbytes));
   hc_snapshot* sn = nullptr;
-  for (auto& k : c->snaps)
-    if (!sn && k && k->bytes >= nbytes) {
-      sn = k;
-      k = nullptr;
-    }
+  {
+    std::lock_guard<std::mutex> lock(c->snaps->m);
+    for (auto& k : c->snaps->kept)
+      if (!sn && k && k->bytes >= nbytes) {
+        sn = k;
+        k = nullptr;
+      }
+  }
   if (!sn) {
     sn = new hc_snapshot();
-    sn->c = c;
+    sn->pool = c->snaps;
     sn->bytes = nbytes;
     if (cudaMalloc((void**)&sn->dev, nbytes) != cudaSuccess) {
       cudaGetLastError();
@@ -729,16 +743,18 @@ extern "C" hc_status hc_snapshot_begin(hc_ctx* c, hc_field f, void* host_pinned,
 
 extern "C" hc_status hc_snapshot_end(hc_snapshot* sn) {
   if (!sn) return HC_ERR_ARG;
-  hc_ctx* c = sn->c;
   const cudaError_t e = cudaEventSynchronize(sn->done);
-  if (e == cudaSuccess)
-    for (auto& k : c->snaps)
+  const std::shared_ptr<hc_snap_pool> pool = sn->pool;
+  std::lock_guard<std::mutex> lock(pool->m);
+  if (e == cudaSuccess && pool->ctx)
+    for (auto& k : pool->kept)
       if (!k) {
         k = sn;
         return HC_OK;
       }
   snapshot_free(sn);
-  return hc_cuda(c, e, "snapshot");
+  if (e == cudaSuccess) return HC_OK;
+  return pool->ctx ? hc_cuda(pool->ctx, e, "snapshot") : HC_ERR_CUDA;
 }
 
 // ------------------------------------------------------------------ series

@@ -19,6 +19,8 @@
 #include <stdint.h>
 #include <stddef.h>
 
+#include <memory>
+#include <mutex>
 #include <utility>
 
 #include "../../include/hc_gpu.h"
@@ -229,6 +231,16 @@ constexpr int kMaxFlowShapes = 24;  // launch shapes of k_flow_route the tuner c
 // output step of a run writes side by side
 constexpr int kSnapKeep = 4;
 
+// The ended snapshots of a context whose buffers are used again.  The context
+// and each of its snapshots share it, so a snapshot may be ended by another
+// thread than the context's, and after the context is gone (ctx is null then,
+// and the end frees).
+struct hc_snap_pool {
+  std::mutex m;  // guards the fields below
+  hc_ctx* ctx = nullptr;
+  struct hc_snapshot* kept[kSnapKeep] = {};
+};
+
 struct hc_ctx {
   hc_view v;
   cudaStream_t s;         // the context's stream
@@ -236,7 +248,7 @@ struct hc_ctx {
                           // conditional node's body is captured)
   cudaStream_t s2;
   cudaStream_t s3;         // snapshots to host memory (hc_snapshot_begin)
-  struct hc_snapshot* snaps[kSnapKeep];  // ended snapshots whose buffers are used again
+  std::shared_ptr<hc_snap_pool> snaps;
   cudaStream_t side;       // a second branch of a captured iteration, with
   cudaEvent_t fork, join;  // the events that split and join it
   hc_iter_handles hcur;   // handles of the iteration being captured

@@ -308,8 +308,11 @@ hc_status hc_mass_reset(hc_ctx* ctx);
  * plain layout (elev, water_depth, qx, qy, Vsusptot, Vel, Tau, bedrock,
  * Manning's n, area, ss, edge) in stream order and moves the copy to
  * `host_pinned` (page-locked memory of nbytes) on a side stream, so hc_run
- * may be called again at once; hc_snapshot_end waits for the copy and frees
- * the snapshot.  The host buffer must stay valid until then. */
+ * may be called again at once; hc_snapshot_end waits for the copy and ends
+ * the snapshot, from any thread, before or after its context is destroyed.
+ * The host buffer must stay valid until then.  A context keeps the device
+ * buffers of up to four ended snapshots for its next ones, until it is
+ * destroyed. */
 typedef struct hc_snapshot hc_snapshot;
 hc_status hc_snapshot_begin(hc_ctx* ctx, hc_field f, void* host_pinned, size_t nbytes,
                             hc_snapshot** out);
