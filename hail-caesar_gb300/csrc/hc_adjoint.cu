@@ -512,7 +512,7 @@ struct Dev {
   template <class T> T* as() { return (T*)p; }
 };
 
-cudaError_t dmalloc(Dev& d, size_t bytes) { return cudaMalloc(&d.p, bytes ? bytes : 8); }
+cudaError_t dmalloc(Dev& d, size_t bytes) { return hc_malloc(&d.p, bytes ? bytes : 8); }
 
 double ms_since(std::chrono::steady_clock::time_point t0) {
   return std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();

@@ -101,19 +101,27 @@ __global__ void k_set_max_ts(const hc_view c, hc_dev* d) {
     s.time_step = cfl();
 }
 
+void snapshots_drop(hc_snap_pool& pool);  // the caller holds pool.m
+
 template <class T>
 hc_status dalloc(hc_ctx* c, T** p, size_t count) {
   size_t bytes = count * sizeof(T);
   if (bytes == 0) bytes = sizeof(T);
-  if (c->max_bytes && c->bytes + bytes > c->max_bytes)
-    return hc_fail(c, HC_ERR_NOMEM, "device allocation cap of %zu bytes exceeded", c->max_bytes);
-  cudaError_t e = cudaMalloc((void**)p, bytes);
+  {
+    std::lock_guard<std::mutex> lock(c->snaps->m);
+    if (c->max_bytes && c->bytes + c->snaps->bytes + bytes > c->max_bytes)
+      snapshots_drop(*c->snaps);
+    if (c->max_bytes && c->bytes + bytes > c->max_bytes)
+      return hc_fail(c, HC_ERR_NOMEM, "device allocation cap of %zu bytes exceeded", c->max_bytes);
+    c->bytes += bytes;
+  }
+  cudaError_t e = hc_malloc((void**)p, bytes);
   if (e != cudaSuccess) {
     *p = nullptr;
-    cudaGetLastError();
+    std::lock_guard<std::mutex> lock(c->snaps->m);
+    c->bytes -= bytes;
     return hc_fail(c, HC_ERR_NOMEM, "cudaMalloc(%zu): %s", bytes, cudaGetErrorString(e));
   }
-  c->bytes += bytes;
   return HC_OK;
 }
 
@@ -215,6 +223,7 @@ extern "C" void* hc_stream(hc_ctx* c) { return c ? (void*)c->s : nullptr; }
 
 // ------------------------------------------------------------------ create
 static hc_status free_all(hc_ctx* c);
+static void snapshots_attach(hc_snap_pool* pool);
 static void snapshots_detach(hc_ctx* c);
 
 hc_divisor host_divisor(double b) {
@@ -244,6 +253,7 @@ extern "C" hc_status hc_create(const hc_params* p, size_t max_bytes, hc_ctx** ou
   hc_ctx* c = new hc_ctx();  // all zero
   c->snaps = std::make_shared<hc_snap_pool>();
   c->snaps->ctx = c;
+  snapshots_attach(c->snaps.get());
   c->max_bytes = max_bytes;
   hc_view& v = c->v;
   v.p = *p;
@@ -287,6 +297,7 @@ extern "C" hc_status hc_create(const hc_params* p, size_t max_bytes, hc_ctx** ou
       cudaEventCreateWithFlags(&c->fork, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&c->join, cudaEventDisableTiming) != cudaSuccess) {
     cudaGetLastError();
+    snapshots_detach(c);
     delete c;
     return HC_ERR_CUDA;
   }
@@ -666,9 +677,10 @@ extern "C" hc_status hc_download(hc_ctx* c, hc_field f, void* host, size_t nbyte
 // A field's copy taken in stream order (a device-to-device copy, so the run
 // can go on at once) and moved to pinned host memory on a side stream.
 // A context keeps the buffers and events of up to kSnapKeep ended snapshots
-// for its next ones (freed with it): allocating and freeing them per snapshot,
-// which waits for the device, took 120 us each (four steps member by member at
-// 900 x 1400 with three rasters: 1.48 -> 1.15 ms).
+// for its next ones: allocating and freeing them per snapshot, which waits for
+// the device, took 120 us each (four steps member by member at 900 x 1400 with
+// three rasters: 1.48 -> 1.15 ms).  Kept buffers count under max_bytes, and go
+// with the context or as soon as an allocation does not fit beside them.
 struct hc_snapshot {
   std::shared_ptr<hc_snap_pool> pool;
   double* dev;
@@ -684,14 +696,50 @@ static void snapshot_free(hc_snapshot* sn) {
   delete sn;
 }
 
-// The context goes: its kept buffers are freed, its open snapshots live on.
-static void snapshots_detach(hc_ctx* c) {
-  std::lock_guard<std::mutex> lock(c->snaps->m);
-  c->snaps->ctx = nullptr;
-  for (auto& k : c->snaps->kept) {
+namespace {
+void snapshots_drop(hc_snap_pool& pool) {
+  for (auto& k : pool.kept) {
     snapshot_free(k);
     k = nullptr;
   }
+  pool.bytes = 0;
+}
+
+// the living contexts' pools
+std::mutex g_pools_m;
+std::vector<hc_snap_pool*> g_pools;
+}  // namespace
+
+cudaError_t hc_malloc(void** p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaSuccess) cudaGetLastError();
+  if (e != cudaErrorMemoryAllocation) return e;
+  {
+    std::lock_guard<std::mutex> all(g_pools_m);
+    for (hc_snap_pool* pool : g_pools) {
+      std::lock_guard<std::mutex> lock(pool->m);
+      snapshots_drop(*pool);
+    }
+  }
+  e = cudaMalloc(p, bytes);
+  if (e != cudaSuccess) cudaGetLastError();
+  return e;
+}
+
+static void snapshots_attach(hc_snap_pool* pool) {
+  std::lock_guard<std::mutex> all(g_pools_m);
+  g_pools.push_back(pool);
+}
+
+// The context goes: its kept buffers are freed, its open snapshots live on.
+static void snapshots_detach(hc_ctx* c) {
+  {
+    std::lock_guard<std::mutex> all(g_pools_m);
+    g_pools.erase(std::find(g_pools.begin(), g_pools.end(), c->snaps.get()));
+  }
+  std::lock_guard<std::mutex> lock(c->snaps->m);
+  c->snaps->ctx = nullptr;
+  snapshots_drop(*c->snaps);
 }
 
 extern "C" hc_status hc_snapshot_begin(hc_ctx* c, hc_field f, void* host_pinned, size_t nbytes,
@@ -708,14 +756,14 @@ extern "C" hc_status hc_snapshot_begin(hc_ctx* c, hc_field f, void* host_pinned,
       if (!sn && k && k->bytes >= nbytes) {
         sn = k;
         k = nullptr;
+        c->snaps->bytes -= sn->bytes;
       }
   }
   if (!sn) {
     sn = new hc_snapshot();
     sn->pool = c->snaps;
     sn->bytes = nbytes;
-    if (cudaMalloc((void**)&sn->dev, nbytes) != cudaSuccess) {
-      cudaGetLastError();
+    if (hc_malloc((void**)&sn->dev, nbytes) != cudaSuccess) {
       snapshot_free(sn);
       return hc_fail(c, HC_ERR_NOMEM, "snapshot buffer");
     }
@@ -746,10 +794,13 @@ extern "C" hc_status hc_snapshot_end(hc_snapshot* sn) {
   const cudaError_t e = cudaEventSynchronize(sn->done);
   const std::shared_ptr<hc_snap_pool> pool = sn->pool;
   std::lock_guard<std::mutex> lock(pool->m);
-  if (e == cudaSuccess && pool->ctx)
+  const hc_ctx* c = pool->ctx;
+  if (e == cudaSuccess && c &&
+      (!c->max_bytes || c->bytes + pool->bytes + sn->bytes <= c->max_bytes))
     for (auto& k : pool->kept)
       if (!k) {
         k = sn;
+        pool->bytes += sn->bytes;
         return HC_OK;
       }
   snapshot_free(sn);

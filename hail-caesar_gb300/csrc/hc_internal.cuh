@@ -239,7 +239,12 @@ struct hc_snap_pool {
   std::mutex m;  // guards the fields below
   hc_ctx* ctx = nullptr;
   struct hc_snapshot* kept[kSnapKeep] = {};
+  size_t bytes = 0;  // of the kept ones' buffers, part of what max_bytes caps
 };
+
+// cudaMalloc; where memory is short, once more without any context's kept
+// snapshot buffers
+cudaError_t hc_malloc(void** p, size_t bytes);
 
 struct hc_ctx {
   hc_view v;
@@ -254,7 +259,7 @@ struct hc_ctx {
   hc_iter_handles hcur;   // handles of the iteration being captured
   int device;
   char err[512];
-  size_t bytes, max_bytes;
+  size_t bytes, max_bytes;  // (bytes: guarded by snaps->m)
   hc_dev *dev;       // device control block
   hc_dev *hdev;      // pinned host mirror
   double *h_elev;    // pinned host buffer (drainage area)

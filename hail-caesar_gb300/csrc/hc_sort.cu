@@ -493,7 +493,7 @@ template <typename T>
 cudaError_t grow(T** p, size_t n) {
   if (*p) cudaFree(*p);
   *p = nullptr;
-  return cudaMalloc((void**)p, std::max<size_t>(n, 1) * sizeof(T));
+  return hc_malloc((void**)p, std::max<size_t>(n, 1) * sizeof(T));
 }
 
 }  // namespace
@@ -652,8 +652,8 @@ extern "C" hc_status hc_drainage_sort(const double* values, uint64_t n, uint32_t
   bool fallback = false;
   int64_t launches = 0;
   cudaError_t e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&dv, n * sizeof(double));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&dp, n * sizeof(uint32_t));
+  if (e == cudaSuccess) e = hc_malloc((void**)&dv, n * sizeof(double));
+  if (e == cudaSuccess) e = hc_malloc((void**)&dp, n * sizeof(uint32_t));
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(dv, values, n * sizeof(double), cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) e = device_sort_values(w, dv, n, dp, s, &fallback, &launches);

@@ -73,7 +73,7 @@ hc_status autotune(hc_ctx* c, bool force) {
     sv.fields.push_back({v.vd, 4 * N2});
   }
   for (auto& f : sv.fields) sv.total += f.second;
-  if (cudaMalloc(&sv.copy, sv.total * 8) != cudaSuccess) {
+  if (hc_malloc((void**)&sv.copy, sv.total * 8) != cudaSuccess) {
     cudaGetLastError();
     return HC_OK;  // no room to tune: keep the shape
   }
@@ -101,7 +101,7 @@ hc_status autotune(hc_ctx* c, bool force) {
   // case that does not occur.
   void* flush = nullptr;
   size_t flush_bytes = 192u << 20;
-  if (cudaMalloc(&flush, flush_bytes) != cudaSuccess) {
+  if (hc_malloc((void**)&flush, flush_bytes) != cudaSuccess) {
     cudaGetLastError();
     flush = nullptr;
   }

@@ -311,8 +311,9 @@ hc_status hc_mass_reset(hc_ctx* ctx);
  * may be called again at once; hc_snapshot_end waits for the copy and ends
  * the snapshot, from any thread, before or after its context is destroyed.
  * The host buffer must stay valid until then.  A context keeps the device
- * buffers of up to four ended snapshots for its next ones, until it is
- * destroyed. */
+ * buffers of up to four ended snapshots for its next ones (within max_bytes;
+ * an open snapshot's buffer is not counted), until it is destroyed or an
+ * allocation of any context does not fit beside them. */
 typedef struct hc_snapshot hc_snapshot;
 hc_status hc_snapshot_begin(hc_ctx* ctx, hc_field f, void* host_pinned, size_t nbytes,
                             hc_snapshot** out);
