@@ -1,5 +1,7 @@
 """Kept snapshot buffers count under a context's max_bytes, make room for its
 other allocations, and go with the context."""
+import functools
+
 import pytest
 
 import synth
@@ -9,10 +11,15 @@ NAMES = ["water_depth", "elev", "qx", "qy", "edge", "Tau"]
 SIDE = 600
 
 
+@functools.lru_cache(maxsize=None)
+def case():
+    return synth.catchment_case(n=SIDE, DX=20.0, hours=24, relief=60.0, hydro_only=True,
+                                lateral=False, storm_start_h=0.2)
+
+
 def make(cap=0):
     import hc
-    return hc.Model(synth.catchment_case(n=SIDE, DX=20.0, hours=24, relief=60.0, hydro_only=True,
-                                         lateral=False, storm_start_h=0.2), max_bytes=cap)
+    return hc.Model(case(), max_bytes=cap)
 
 
 def smallest_cap():
