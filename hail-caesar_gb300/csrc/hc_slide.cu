@@ -876,6 +876,7 @@ __global__ void __launch_bounds__(32 * kCreepWarps) k_creep_grain(const hc_view 
           }
           __threadfence();
         }
+        __syncwarp();  // the other lanes' reads come after lane 0's fence
         seen = __shfl_sync(kFull, got, 0);
         if (seen < 0) {  // gave up: the records are not complete
           if (L == 0) {
