@@ -849,7 +849,7 @@ static hc_status device_error(hc_ctx* c) {
   const int e = c->hdev->err_code;
   if (e == 301) return hc_fail(c, HC_ERR_NONFINITE, "non-finite water depth (device error 301)");
   if (e == 401) return hc_fail(c, HC_ERR_TIMEOUT, "drainage sweep: a device wait gave up (401)");
-  if (e == 402) return hc_fail(c, HC_ERR_TIMEOUT, "creep: a device wait gave up (402)");
+  if (e == 402) return hc_fail(c, HC_ERR_TIMEOUT, "creep: a device wait gave up (402); the creep is complete");
   return hc_fail(c, HC_ERR_STATE, "device error %d", e);
 }
 
@@ -1127,13 +1127,26 @@ extern "C" hc_status hc_global_landsliding(hc_ctx* c, int32_t* sweeps) {
   return HC_OK;
 }
 
+// After run_creep and a pull.  A wait that ran out left nothing undone: the
+// status tells of it, and the context goes on.
+static hc_status creep_status(hc_ctx* c) {
+  hc_dev* hd = c->hdev;
+  if (!(hd->pause & HC_PAUSE_ERROR)) return HC_OK;
+  const hc_status st = device_error(c);
+  if (hd->err_code == 402) {
+    hd->err_code = 0;
+    hd->pause &= ~HC_PAUSE_ERROR;
+    HC_TRY(push(c));
+  }
+  return st;
+}
+
 extern "C" hc_status hc_creep(hc_ctx* c, double time) {
   if (!c) return HC_ERR_ARG;
   if (c->v.p.hydro_only) return hc_fail(c, HC_ERR_STATE, "erosion arrays absent (hydro_only)");
   HC_TRY(run_creep(c, time));
   HC_TRY(pull(c));
-  if (c->hdev->pause & HC_PAUSE_ERROR) return device_error(c);
-  return HC_OK;
+  return creep_status(c);
 }
 
 // ------------------------------------------------------------------ hc_run
@@ -1336,6 +1349,7 @@ static hc_status finish_iteration(hc_ctx* c, int flags) {
 static hc_status host_steps(hc_ctx* c, int flags) {
   hc_dev* hd = c->hdev;
   const hc_params& p = c->v.p;
+  hc_status gave_up = HC_OK;  // of a creep that is complete: the other steps still run
   if (hd->pause & HC_PAUSE_HOSTSTEP) {
     hd->pause &= ~HC_PAUSE_HOSTSTEP;
     if (!p.hydro_only && !(flags & HC_RUN_NOHILL)) {
@@ -1345,6 +1359,8 @@ static hc_status host_steps(hc_ctx* c, int flags) {
         HC_TRY(push(c));
         HC_TRY(run_creep(c, p.creep_coeff));
         HC_TRY(pull(c));
+        gave_up = creep_status(c);
+        if (gave_up != HC_OK && gave_up != HC_ERR_TIMEOUT) return gave_up;
       }
       if (hd->s.cycle > hd->s.creep_time2) {  // call_global_landsliding :1986
         StatTimer st(c, HC_STAT_GLOBAL_SLIDE);
@@ -1352,6 +1368,7 @@ static hc_status host_steps(hc_ctx* c, int flags) {
         HC_TRY(push(c));
         HC_TRY(run_global_landsliding(c, nullptr));
         HC_TRY(pull(c));
+        if (hd->pause & HC_PAUSE_ERROR) return device_error(c);
       }
     }
     HC_TRY(push(c));
@@ -1362,7 +1379,7 @@ static hc_status host_steps(hc_ctx* c, int flags) {
     HC_TRY(push(c));
     HC_TRY(recompute_points(c, true));
   }
-  return HC_OK;
+  return gave_up;
 }
 
 // hc_run in pieces, so that hc_run_ensemble can keep several contexts' graphs
@@ -1436,7 +1453,10 @@ static hc_status run_after_chunk(hc_ctx* c, int32_t flags, bool* finished) {
   c->launches += turns * c->graph_kernels + (int64_t)(hd->body_kernels - c->body_k0);
   c->stat_n[HC_STAT_IDLE_ITERS] += turns * K - its;
   if (hd->pause & HC_PAUSE_ERROR) return device_error(c);
-  if (hd->pause & (HC_PAUSE_ERODE | HC_PAUSE_LATERAL)) HC_TRY(finish_iteration(c, flags));
+  if (hd->pause & (HC_PAUSE_ERODE | HC_PAUSE_LATERAL)) {
+    HC_TRY(finish_iteration(c, flags));
+    if (hd->pause & HC_PAUSE_ERROR) return device_error(c);
+  }
   HC_TRY(host_steps(c, flags));
   if ((hd->pause & HC_PAUSE_FINISHED) || hd->budget <= 0) {
     *finished = true;

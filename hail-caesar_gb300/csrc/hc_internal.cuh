@@ -210,9 +210,9 @@ struct hc_view {
   double *vpart; int vpart_cap;  // per-block partial sums (grid_sum, scan_area's volume)
   hc_step_record *rec; int64_t rec_cap;
   // test hook of the bounded device waits (hc_test_bounded_waits): when
-  // wait_spins > 0 the drainage sweep's waits give up after that many spins,
-  // and it expects barrier_extra cells more than there are, so that they run
-  // out
+  // wait_spins > 0 the waits of the drainage sweep and of creep's rows give up
+  // after that many spins, and expect barrier_extra cells or columns more than
+  // there are, so that they run out
   int wait_spins, barrier_extra;
 };
 

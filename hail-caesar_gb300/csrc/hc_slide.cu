@@ -710,7 +710,10 @@ __global__ void k_creep_gather(const hc_view c, double* tempcreep, double time) 
 // visit comes after all earlier ones that it conflicts with, and the records
 // are the serial loop's.  Rows are handed out in order by a counter, so the
 // topmost unfinished row is always held by a running warp and never waits
-// for one that is not; every wait is bounded all the same.
+// for one that is not; every wait is bounded all the same.  Where one runs
+// out, the warps leave, each row at the column it had come to, and a second
+// launch of one warp finishes the rows in order, without a wait (rest): the
+// records are the serial loop's then too, and error 402 tells of it.
 //
 // Within a visit lane n holds fraction n of the records (the serial sums over
 // the fractions keep their order: every lane forms the same sum), and the
@@ -838,37 +841,45 @@ static __device__ void creep_slide(const hc_view& c, size_t acell, double& a, do
 
 __global__ void __launch_bounds__(32 * kCreepWarps) k_creep_grain(const hc_view c, hc_dev* d,
                                                                   CreepSync* sync, uint8_t* made,
-                                                                  double time) {
+                                                                  double time, int rest) {
   const int cx[8] = {0, 1, 1, 1, 0, -1, -1, -1};
   const int cy[8] = {-1, -1, 0, 1, 1, 1, 0, -1};
   const int L = threadIdx.x & 31;
   const size_t W = c.W;
   const int last = c.jmax - 1;
-  for (;;) {
-    unsigned ticket = 0;
-    if (L == 0) ticket = atomicAdd(&sync->ticket, 1u);
-    ticket = __shfl_sync(kFull, ticket, 0);
-    if (ticket >= (unsigned)(c.imax - 2)) return;
+  if (rest && sync->err == 0) return;
+  // a test shortens the waits and has them run out: no row reaches `beyond`
+  const long limit = c.wait_spins > 0 ? (long)c.wait_spins : kCreepSpins;
+  const int beyond = c.wait_spins > 0 ? c.barrier_extra : 0;
+  for (unsigned row = 0;; row++) {
+    unsigned ticket = row;
+    if (!rest) {
+      if (L == 0) ticket = atomicAdd(&sync->ticket, 1u);
+      ticket = __shfl_sync(kFull, ticket, 0);
+    }
+    if (ticket >= (unsigned)(c.imax - 2)) break;
     const int x = 2 + (int)ticket;
     const volatile int* above = &sync->done[x - 1];
     volatile int* mine = &sync->done[x];
-    int seen = (x == 2) ? INT_MAX : 0;  // last column the row above is known to have visited
+    // last column the row above is known to have visited
+    int seen = (x == 2 || rest) ? INT_MAX : 0;
     double v = -1;
     unsigned moves = 0;
-    for (int y = 2; y <= last; y++) {
+    const int first = rest ? max(2, *mine + 1) : 2;
+    for (int y = first; y <= last; y++) {
       const int q = (y - 2) & 3;
-      if (q == 0) {  // the moves of cells y .. y+3
-        const int yy = y + (L >> 3);
+      if (q == 0 || y == first) {  // the moves of four cells, y - q ..
+        const int yy = y - q + (L >> 3);
         v = yy <= last ? creep_temp(c, x, yy, L & 7, time) : -1.0;
         moves = __ballot_sync(kFull, v >= 0);
       }
-      const int need = min(y + 2, last);
+      const int need = min(y + 2, last) + beyond;
       if (seen < need) {
         int got = 0;
         if (L == 0) {
           long spins = 0;
           while ((got = *above) < need) {
-            if (++spins > kCreepSpins || *(volatile unsigned*)&sync->err) {
+            if (++spins > limit || *(volatile unsigned*)&sync->err) {
               atomicExch(&sync->err, 1u);
               got = -1;
               break;
@@ -878,13 +889,7 @@ __global__ void __launch_bounds__(32 * kCreepWarps) k_creep_grain(const hc_view 
         }
         __syncwarp();  // the other lanes' reads come after lane 0's fence
         seen = __shfl_sync(kFull, got, 0);
-        if (seen < 0) {  // gave up: the records are not complete
-          if (L == 0) {
-            d->err_code = 402;
-            atomicOr((unsigned int*)&d->pause, HC_PAUSE_ERROR);
-          }
-          return;
-        }
+        if (seen < 0) return;  // gave up
       }
       const unsigned m = (moves >> (8 * q)) & 0xffu;
       const size_t cell = (size_t)x * W + y;
@@ -920,6 +925,10 @@ __global__ void __launch_bounds__(32 * kCreepWarps) k_creep_grain(const hc_view 
       }
       if (L == 0) *mine = y;
     }
+  }
+  if (rest && L == 0) {
+    d->err_code = 402;
+    d->pause |= HC_PAUSE_ERROR;
   }
 }
 
@@ -1098,11 +1107,12 @@ hc_status run_creep(hc_ctx* c, double time) {
     cudaMemsetAsync(sync, 0, sizeof(CreepSync) + (size_t)(c->v.imax + 2) * sizeof(int), c->s);
     cudaMemsetAsync(sc.flag, 0, n, c->s);
     k_creep_grain<<<(rows + kCreepWarps - 1) / kCreepWarps, 32 * kCreepWarps, 0, c->s>>>(
-        c->v, c->dev, sync, sc.flag, time);
+        c->v, c->dev, sync, sc.flag, time, 0);
+    k_creep_grain<<<1, 32, 0, c->s>>>(c->v, c->dev, sync, sc.flag, time, 1);
     k_flag_count<<<nblocks, 1024, 0, c->s>>>(sc.flag, n, sc.block_sums, sc.count, c->dev, 0);
     k_creep_number<<<nblocks, 1024, 0, c->s>>>(c->v, c->dev, sc.flag, sc.block_sums);
     k_creep_total<<<1, 1, 0, c->s>>>(c->dev, sc.count);
-    count_launch(c, 4);
+    count_launch(c, 5);
   }
   k_creep_apply<<<g, b, 0, c->s>>>(c->v, tempcreep);
   count_launch(c, 1);

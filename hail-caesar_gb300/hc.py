@@ -230,8 +230,9 @@ class Model:
         return {k: getattr(m, k) for k, _ in hc_mass._fields_}
 
     def test_bounded_waits(self, spins, extra_arrivals=1):
-        """Shortens the drainage sweep's device waits and makes them run out
-        (spins 0: back to normal); see hc_test_bounded_waits."""
+        """Shortens the device waits of the drainage sweep and of creep and
+        makes them run out (spins 0: back to normal); see
+        hc_test_bounded_waits."""
         self._check(self.lib.hc_test_bounded_waits(self.h, spins, extra_arrivals),
                     "test_bounded_waits")
 

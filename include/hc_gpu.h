@@ -388,13 +388,15 @@ hc_status hc_get_run_stats(hc_ctx* ctx, int64_t* counts, double* host_ms, int32_
 
 /* Test hook of the bounded device waits (no counterpart in the reference).
  * The drainage recomputation (drainage_area_D8 :2091-2271) runs as one
- * kernel whose warps wait for cells that others release;
- * every such wait gives up after a bounded number of spins, and the call
- * that launched it returns HC_ERR_TIMEOUT with the context still usable (hc_run
- * then redoes the recomputation first thing in its next call).  spins > 0
- * sets that bound (0 restores the built-in one) and makes the kernel expect
- * extra_arrivals more cells than there are, so that the waits run out: the
- * way the tests check this path without a fault. */
+ * kernel whose warps wait for cells that others release, creep's grain
+ * transfers (:5293-5427) as one whose rows wait for the row above; every such
+ * wait gives up after a bounded number of spins, and the call that launched it
+ * returns HC_ERR_TIMEOUT with the context still usable: hc_run redoes the
+ * drainage recomputation first thing in its next call, and creep is finished
+ * without waits before the call returns.  spins > 0 sets that bound (0
+ * restores the built-in one) and makes the kernels expect extra_arrivals more
+ * cells, or columns, than there are, so that the waits run out: the way the
+ * tests check this path without a fault. */
 hc_status hc_test_bounded_waits(hc_ctx* ctx, int32_t spins, int32_t extra_arrivals);
 
 /* Launch-shape autotuner (no counterpart in the reference).  hc_run times

@@ -53,3 +53,63 @@ def test_many_rows(gpu_lib, oracle_mod, imax, jmax):
     m.creep(5.0)
     o.lib.hco_creep(o.h, 5.0)
     check(m, o)
+
+
+@pytest.mark.parametrize("imax,jmax", [(4, 3), (5, 40), (40, 5), (70, 33)])
+@pytest.mark.parametrize("spins,beyond", [(1, 1), (40, 1), (3000, 7), (1, 0)])
+def test_waits_run_out(gpu_lib, oracle_mod, imax, jmax, spins, beyond):
+    """A wait that gives up is reported, and the creep is complete all the
+    same; so is the next one, with the built-in bound."""
+    import hc
+    m, o = creep_case(imax, jmax, oracle_mod)
+    m.test_bounded_waits(spins, beyond)
+    if beyond:  # the row above never gets there
+        with pytest.raises(hc.HCError, match="HC_ERR_TIMEOUT"):
+            m.creep(5.0)
+    else:  # one look at the row above may or may not be enough
+        try:
+            m.creep(5.0)
+        except hc.HCError as e:
+            assert "HC_ERR_TIMEOUT" in str(e)
+    o.lib.hco_creep(o.h, 5.0)
+    check(m, o)
+    m.test_bounded_waits(0, 0)
+    m.creep(5.0)
+    o.lib.hco_creep(o.h, 5.0)
+    check(m, o)
+
+
+@pytest.mark.parametrize("after", [0, 5])
+def test_wait_runs_out_in_a_run(gpu_lib, after):
+    """A creep that falls due in a call's last iteration (as always where a
+    program runs one iteration a call), or `after` iterations before it: the
+    call returns HC_ERR_TIMEOUT after that iteration, and the next one goes on
+    as a run that never timed out."""
+    import hc
+    case = synth.catchment_case(n=48, DX=20.0, hours=72, relief=60.0, hydro_only=False,
+                                lateral=False, storm_start_h=0.5)
+    case.params.creep_time_interval = 60
+    n = 600
+    ref = hc.Model(case)
+    cycle0 = ref.scalars().cycle
+    ra = ref.run(n)
+    due, at = cycle0, []
+    for k, cycle in enumerate(ra[:, hc.STEP_FIELDS.index("cycle")]):
+        if cycle > due:
+            due += 60
+            at.append(k)
+    assert ref.run_stats()["creep"][0] == len(at) >= 2
+    k = at[-1]
+    assert n - k > 10
+    m = hc.Model(case)
+    m.run(k)
+    assert (m.field("index") != -9999).any(), "no grain to move"
+    m.test_bounded_waits(1, 1)
+    with pytest.raises(hc.HCError, match="HC_ERR_TIMEOUT creep"):
+        m.run(1 + after)
+    assert int(m.scalars().counter) == k + 1
+    m.test_bounded_waits(0, 0)
+    rb = m.run(n - k - 1)
+    assert_bitwise(rb, ra[k + 1:], "records")
+    for f in ("elev", "index", "grain", "strata", "water_depth", "qx", "area"):
+        assert_bitwise(m.field(f), ref.field(f), f)
