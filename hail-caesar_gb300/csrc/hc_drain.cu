@@ -307,6 +307,7 @@ struct DrainSync {
 
 constexpr int kSweepThreads = 128;
 constexpr int kSweepBlocks = 2;  // per multiprocessor
+constexpr unsigned kReportTurns = 256;  // about half a millisecond
 constexpr int kSpareMax = 32 * 8;  // per lane: 8 released but one it keeps, and a queue entry
 
 // the first frontier's cells, as queue entries
@@ -386,7 +387,7 @@ __global__ void __launch_bounds__(kSweepThreads) k_drain_sweep(const hc_view c, 
   const unsigned lane = threadIdx.x & 31;
   const int W = (int)c.W;
   const bool test = c.wait_spins > 0;  // a test shortens the waits and has them run out
-  const long limit = test ? (long)c.wait_spins : (1L << 24);
+  const unsigned limit = test ? (unsigned)c.wait_spins : 1u << 24;
   const unsigned long long M =
       (unsigned long long)c.imax * c.jmax + (test ? (unsigned)c.barrier_extra : 0u);
   uint32_t cell = 0;             // 0: none (cell 0 is a padding cell)
@@ -395,7 +396,11 @@ __global__ void __launch_bounds__(kSweepThreads) k_drain_sweep(const hc_view c, 
   unsigned slot = 0;
   bool ticket = false;           // the lane waits for queue entry `slot`
   unsigned finished = 0;         // cells finished by the lane since the last report
-  long idle = 0;
+  unsigned turn = 0;
+  unsigned waited = 0;           // turns the lane has waited for its cell's areas
+  // lane 0: the cells finished when it last looked, and its looks since then
+  unsigned long long done = 0;
+  unsigned idle = 0;
   __shared__ uint4 spare[kSweepThreads / 32][kSpareMax];  // released: cell, hop, head
   uint4* mine = spare[threadIdx.x >> 5];
   unsigned out0 = 0, out1 = 0;   // of them, [out0, out1) go to the queue ...
@@ -457,9 +462,10 @@ __global__ void __launch_bounds__(kSweepThreads) k_drain_sweep(const hc_view c, 
       rel &= rel - 1;  // the lane goes on with the lowest of them itself
       next_hop = hop + 1;
       finished++;
+      waited = 0;
       most = max(most, hop);
     } else if (cell != 0) {
-      idle++;  // an area still on its way
+      waited++;  // an area still on its way
     }
     // the lane's queue entry: its own when it is idle (it may have been given
     // a cell by another lane since it took its number), else one more to share
@@ -525,28 +531,38 @@ __global__ void __launch_bounds__(kSweepThreads) k_drain_sweep(const hc_view c, 
         ticket = true;
       }
     }
-    if (out1 == out0 && !__any_sync(FULL, cell != 0)) {
-      // nothing to do: report, and leave when every cell is finished
+    // Report what was finished: with nothing to do, and every kReportTurns
+    // turns of work, so that the warps that wait see the sweep move.  With
+    // nothing to do, leave when every cell is finished, or when none was for
+    // as many looks as the bound allows.
+    const bool quiet = out1 == out0 && !__any_sync(FULL, cell != 0);
+    if (quiet || ++turn == kReportTurns) {
+      turn = 0;
       unsigned f = finished;
       for (int o = 16; o > 0; o >>= 1) f += __shfl_xor_sync(FULL, f, o);
       finished = 0;
       unsigned stop = 0;
       if (lane == 0) {
         if (f) atomicAdd(&g->done, (unsigned long long)f);
-        if (ld_relaxed(&g->done) >= M) {
-          stop = 1;
-        } else if (++idle > limit || *(volatile unsigned*)&g->err) {
-          atomicExch(&g->err, 1u);
-          stop = 1;
-        } else {
-          __nanosleep(64);
+        if (quiet) {
+          const unsigned long long now = ld_relaxed(&g->done);
+          if (now != done) idle = 0;
+          done = now;
+          if (now >= M) {
+            stop = 1;
+          } else if (++idle > limit || *(volatile unsigned*)&g->err) {
+            atomicExch(&g->err, 1u);
+            stop = 1;
+          } else {
+            __nanosleep(64);
+          }
         }
       }
+      if (__any_sync(FULL, waited > limit)) {
+        if (lane == 0) atomicExch(&g->err, 1u);
+        break;
+      }
       if (__shfl_sync(FULL, stop, 0)) break;
-    }
-    if (__any_sync(FULL, idle > limit)) {
-      if (lane == 0) atomicExch(&g->err, 1u);
-      break;
     }
   }
   for (int o = 16; o > 0; o >>= 1) most = max(most, __shfl_xor_sync(FULL, most, o));
