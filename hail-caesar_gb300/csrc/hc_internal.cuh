@@ -122,9 +122,12 @@ struct hc_drain_aux {
 };
 
 // A divisor prepared for ddiv_by (below): its significand, exponent and a
-// 64-bit reciprocal of the significand.
+// 64-bit reciprocal of the significand.  V is floor(2^116/mb), or a few
+// units less where the device formed it, so its top bit is set; for
+// mb == 2^52, where that floor has 65 bits, it is taken as 2^64 - 1.  V = 0
+// asks for the hardware division.
 struct hc_divisor {
-  unsigned long long mb, V;  // significand of b, ~2^116/mb (unused when mb == 2^52)
+  unsigned long long mb, V;  // significand of b, reciprocal
   double b;
   int eb;                    // biased exponent of b
   int ok;                    // b normal and finite
@@ -662,7 +665,7 @@ HC_DEV double ddiv_by(double a, const hc_divisor& d) {
   const int less = ma < mb ? 1 : 0;
   ma <<= less;
   const int er = ea - d.eb + 1023 - less;
-  // (a divisor prepared elsewhere may hold no V for a power of two)
+  // (V = 0: a divisor prepared without a reciprocal)
   if (!d.ok || (unsigned)(ea - 1) >= 2046u || (unsigned)(er - 1) >= 2045u ||
       (long long)d.V >= 0) {
     // a zero dividend (frequent: flat water surfaces, cells with no net
@@ -682,7 +685,8 @@ HC_DEV double ddiv_by(double a, const hc_divisor& d) {
 
 HC_DEV double ddiv_rn(double a, double b) { return ddiv_by(a, ddiv_prep(b)); }
 
-// hc_divisor for a divisor fixed for the run, V exact (floor(2^116/mb))
+// hc_divisor for a divisor fixed for the run, V exact (floor(2^116/mb), and
+// 2^64 - 1 for a power of two)
 hc_divisor host_divisor(double b);
 
 // (double)f on the integer pipe for normal floats and zeros, the conversion
