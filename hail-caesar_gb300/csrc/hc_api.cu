@@ -315,9 +315,10 @@ extern "C" hc_status hc_create(const hc_params* p, size_t max_bytes, hc_ctx** ou
   // partial sums: one per block of scan_area (32 x 8 cells) or of a grid_sum
   v.vpart_cap = (int)std::max<size_t>(
       (size_t)((p->jmax + 31) / 32) * (size_t)((p->imax + 7) / 8), 152 * 8);
-  A(v.vpart, (size_t)v.vpart_cap) A(v.flux, 4 * ((size_t)p->imax + p->jmax))
-  A(v.drain_pos, N2) A(v.drain_f0, N2) A(v.drain_f1, N2) A(v.drain_pend, N2) A(v.drain_dt, N2)
+  A(v.vpart, (size_t)v.vpart_cap)
+  A(v.drain_pos, N2) A(v.drain_pend, N2) A(v.drain_dt, N2)
   A(v.drain_share, 8 * N2) A(v.drain_head, N2)
+  v.flux = v.drain_share;
   A(v.drain_aux, 1)
   if (sed) {
     A(v.sflux, 40 * N2) A(v.sdirty, N2) A(v.grain, kGrainStride * N2)
@@ -405,9 +406,9 @@ static hc_status free_all(hc_ctx* c) {
   void* ptrs[] = {v.elev, v.h, v.qx, v.qy, v.qxs, v.qys, v.vs, v.vel, v.tau, v.bed, v.man, v.man2,
                   v.area, v.ss, v.vd, v.sflux, v.grain, v.strata, v.index, v.mask, v.rfarea,
                   v.edge, v.edge2, v.veg, v.cin_x, v.cin_y, v.erodetot, v.erodetot3, v.pre,
-                  v.chains, v.ent_list, v.ent_qs, v.drain_pos, v.drain_f0, v.drain_f1, v.drain_pend, v.drain_dt, v.drain_share, v.drain_head,
+                  v.chains, v.ent_list, v.ent_qs, v.drain_pos, v.drain_pend, v.drain_dt, v.drain_share, v.drain_head,
                   v.drain_snap, v.drain_aux, v.alloc_key, v.red, v.touched, v.topm, v.rain, v.rec, c->dev, v.wet,
-                  v.wet_sums, v.wet_bits, v.vpart, v.flux, v.sdirty, v.border,
+                  v.wet_sums, v.wet_bits, v.vpart, v.sdirty, v.border,
                   v.reach[0], v.reach[1], v.reach[2], extra(c).lateral};
   for (void* q : ptrs)
     if (q) cudaFree(q);

@@ -152,11 +152,11 @@ __global__ void k_drain_pos(const hc_view c, const uint32_t* __restrict__ order)
 
 // per interior cell: the sum of downhill drops (difftot, the
 // reference's clamped 8-neighbour loop in its order), the number of higher
-// neighbours to wait for (cells with none start the first frontier), whether
+// neighbours to wait for, whether
 // the sweep reaches the cell (drain_pos 1/0: below the selected last
 // position, and not the unique lowest cell), and whether two higher
 // neighbours share an elevation
-__global__ void k_drain_init(const hc_view c, hc_dev* d, const double* __restrict__ el) {
+__global__ void k_drain_init(const hc_view c, const double* __restrict__ el) {
   int i, j;
   if (!interior_ij(c, i, j)) return;
   const size_t W = c.W;
@@ -193,16 +193,6 @@ __global__ void k_drain_init(const hc_view c, hc_dev* d, const double* __restric
   const bool reached = !(u > a->prefix) &&
                        !(a->min_u < kZeroKey && a->min_count == 1 && u == a->min_u);
   c.drain_pos[cell] = reached ? 1u : 0u;
-  // one atomic per warp
-  const unsigned act = __activemask(), m = __ballot_sync(act, higher == 0);
-  if (m) {
-    const unsigned lane = threadIdx.x & 31;
-    const int leader = __ffs(act) - 1;
-    unsigned base = 0;
-    if ((int)lane == leader) base = atomicAdd(&d->drain_front, (unsigned)__popc(m));
-    base = __shfl_sync(act, base, leader);
-    if (higher == 0) c.drain_f0[base + __popc(m & ((1u << lane) - 1u))] = (uint32_t)cell;
-  }
 }
 
 // A cell's terms, before the sweep: its higher neighbours that the sweep
@@ -296,7 +286,7 @@ __global__ void __launch_bounds__(256) k_drain_terms(const hc_view c,
   c.area[cell] = bits_d(-1LL);
 }
 
-// The sweep's shared state, all zero at the start but `tail`.
+// The sweep's shared state, all zero at the start.
 struct DrainSync {
   unsigned long long done;  // cells finished
   unsigned int tail;        // queue entries appended
@@ -310,12 +300,41 @@ constexpr int kSweepBlocks = 2;  // per multiprocessor
 constexpr unsigned kReportTurns = 256;  // about half a millisecond
 constexpr int kSpareMax = 32 * 8;  // per lane: 8 released but one it keeps, and a queue entry
 
-// the first frontier's cells, as queue entries
-__global__ void k_drain_seed(const uint32_t* __restrict__ front, DrainSync* g,
-                             unsigned long long* queue) {
-  const unsigned n = g->tail;
-  for (unsigned k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x)
-    queue[k] = (1ull << 32) | front[k];
+// The first frontier's cells (no higher neighbour), as queue entries: a warp
+// takes 32 columns of kSeedRows rows, and a block's eight warps one atomic (a
+// set-up at 1500^2 took 50 us longer with one per warp and row).
+constexpr int kSeedRows = 8;
+
+__global__ void __launch_bounds__(256) k_drain_seed(const hc_view c, DrainSync* g,
+                                                    unsigned long long* queue) {
+  __shared__ unsigned count[8], base;
+  const unsigned lane = threadIdx.x, warp = threadIdx.y;
+  const int j = 1 + blockIdx.x * 32 + lane;
+  const int i0 = 1 + (blockIdx.y * 8 + warp) * kSeedRows;
+  unsigned m[kSeedRows], n = 0;
+#pragma unroll
+  for (int r = 0; r < kSeedRows; r++) {
+    const bool in = i0 + r <= c.imax && j <= c.jmax;
+    m[r] = __ballot_sync(0xffffffffu, in && c.drain_pend[(size_t)(i0 + r) * c.W + j] == 0);
+    n += __popc(m[r]);
+  }
+  if (lane == 0) count[warp] = n;
+  __syncthreads();
+  if (lane == 0 && warp == 0) {
+    unsigned all = 0;
+    for (int w = 0; w < 8; w++) all += count[w];
+    base = all ? atomicAdd(&g->tail, all) : 0u;
+  }
+  __syncthreads();
+  unsigned at = base;
+  for (unsigned w = 0; w < warp; w++) at += count[w];
+#pragma unroll
+  for (int r = 0; r < kSeedRows; r++) {
+    if ((m[r] >> lane) & 1u)
+      queue[at + __popc(m[r] & ((1u << lane) - 1u))] =
+          (1ull << 32) | (uint32_t)((size_t)(i0 + r) * c.W + j);
+    at += __popc(m[r]);
+  }
 }
 
 __device__ __forceinline__ unsigned long long ld_relaxed(const void* p) {
@@ -573,7 +592,6 @@ __global__ void __launch_bounds__(kSweepThreads) k_drain_sweep(const hc_view c, 
 __global__ void k_drain_end(hc_dev* d, const DrainSync* g) {
   d->drain_done = (unsigned)g->done;
   d->drain_levels = g->hops;
-  d->drain_front = 0;
   if (g->err) {
     d->err_code = 401;
     d->pause |= HC_PAUSE_ERROR;
@@ -755,7 +773,7 @@ hc_status run_drainage_device(hc_ctx* c, const double* el, bool area_valid,
       k_sel_hist<<<g, b, 0, s>>>(v, el, shift);
       k_sel_pick<<<1, 256, 0, s>>>(v, shift, P);
     }
-    k_drain_init<<<g, b, 0, s>>>(v, c->dev, el);
+    k_drain_init<<<g, b, 0, s>>>(v, el);
     c->launches += 19;
     hc_drain_aux a;
     if (cudaMemcpyAsync(&a, v.drain_aux, sizeof a, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
@@ -766,9 +784,10 @@ hc_status run_drainage_device(hc_ctx* c, const double* el, bool area_valid,
     const bool bottom_ok =
         a.min_u > kZeroKey || (a.min_u < kZeroKey && (a.min_count == 1 || !a.min_matters));
     if (a.contrib_tie || !top_ok || !bottom_ok) {
-      if (sort_order(c, el, v.drain_f1) != HC_OK) return HC_ERR_CUDA;
+      uint32_t* order = (uint32_t*)v.drain_share;  // free until the terms are formed
+      if (sort_order(c, el, order) != HC_OK) return HC_ERR_CUDA;
       if (cudaMemsetAsync(v.drain_pos, 0, N2 * 4, s) != cudaSuccess) return HC_ERR_CUDA;
-      k_drain_pos<<<152 * 4, 256, 0, s>>>(v, v.drain_f1);
+      k_drain_pos<<<152 * 4, 256, 0, s>>>(v, order);
       c->launches += 1;
       *sorted = true;
     }
@@ -778,13 +797,12 @@ hc_status run_drainage_device(hc_ctx* c, const double* el, bool area_valid,
     static_assert(sizeof(DrainSync) <= sizeof(hc_drain_aux::hist), "sweep state fits");
     DrainSync* gs = (DrainSync*)((char*)v.drain_aux + offsetof(hc_drain_aux, hist));
     unsigned long long* queue = (unsigned long long*)v.drain_dt;
-    const unsigned* front = (const unsigned*)((const char*)c->dev + offsetof(hc_dev, drain_front));
     if (cudaMemsetAsync(gs, 0, sizeof(DrainSync), s) != cudaSuccess ||
-        cudaMemsetAsync(queue, 0, N2 * 8, s) != cudaSuccess ||
-        cudaMemcpyAsync((char*)gs + offsetof(DrainSync, tail), front, sizeof(unsigned),
-                        cudaMemcpyDeviceToDevice, s) != cudaSuccess)
+        cudaMemsetAsync(queue, 0, N2 * 8, s) != cudaSuccess)
       return HC_ERR_CUDA;
-    k_drain_seed<<<c->sms, 256, 0, s>>>(v.drain_f0, gs, queue);
+    const int seed_rows = 8 * kSeedRows;
+    k_drain_seed<<<dim3((v.jmax + 31) / 32, (v.imax + seed_rows - 1) / seed_rows), b, 0, s>>>(
+        v, gs, queue);
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);

@@ -86,7 +86,7 @@ struct hc_dev {
   unsigned long long body_kernels;  // kernels run inside conditional graph nodes
   int wet_count;          // length of hc_view::wet
   int do_drain;           // this iteration moved the baseflow threshold
-  unsigned int drain_front, drain_done, drain_points, drain_levels;
+  unsigned int drain_done, drain_points, drain_levels;
   unsigned int drain_rf[HC_MAX_RF + 1];
   int adj_mode;           // 0 off, 1 record the time steps, 2 impose them
   int64_t adj_i, adj_n;   // next iteration, capacity of hc_view::adj_dt
@@ -187,12 +187,14 @@ struct hc_view {
   uint32_t *chains;              // 4 * N2: apply-pass chain starts (x pass, y pass), then
                                  // the resume points of long chains (x, y)
   // drainage area (hc_drain.cu): sweep position, sum of drops (then the
-  // sweep's queue), higher neighbours pending, the first frontier, the sort's
-  // order, and the elevation snapshot
-  uint32_t *drain_pos, *drain_f0, *drain_f1;
+  // sweep's queue), higher neighbours pending, and the elevation snapshot
+  uint32_t *drain_pos;
   int32_t *drain_pend;
   double *drain_dt, *drain_snap;
-  double *drain_share;    // 8*N2: a cell's shares of its higher neighbours' areas, in sweep order
+  // 8*N2: a cell's shares of its higher neighbours' areas, in sweep order (the
+  // sort's order before the shares are formed).  Between recomputations it is
+  // scratch: water_flux_out's terms, the progress of creep's rows.
+  double *drain_share;
   unsigned long long *drain_head;  // N2: which neighbours they are, and the lower ones
   struct hc_drain_aux *drain_aux;
   // adjoint runs (hc_adjoint.cu): per-iteration time steps, recorded or
@@ -210,6 +212,7 @@ struct hc_view {
   double *red;                   // reduction scratch
   int32_t *scan_tmp;             // scan scratch
   double *flux;                  // water_flux_out: 2 * (2 imax + 2 jmax) edge-cell terms
+                                 // (in drain_share)
   double *vpart; int vpart_cap;  // per-block partial sums (grid_sum, scan_area's volume)
   hc_step_record *rec; int64_t rec_cap;
   // test hook of the bounded device waits (hc_test_bounded_waits): when

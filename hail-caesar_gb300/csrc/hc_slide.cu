@@ -1102,8 +1102,8 @@ hc_status run_creep(hc_ctx* c, double time) {
     SlideScratch sc = slide_scratch(c);
     const size_t n = c->v.N2;
     const int nblocks = (int)((n + 1023) / 1024), rows = c->v.imax - 2;
-    // the rows' progress lives in the drainage frontier, which is idle here
-    CreepSync* sync = (CreepSync*)c->v.drain_f0;
+    // the rows' progress lives in the drainage shares, which are idle here
+    CreepSync* sync = (CreepSync*)c->v.drain_share;
     cudaMemsetAsync(sync, 0, sizeof(CreepSync) + (size_t)(c->v.imax + 2) * sizeof(int), c->s);
     cudaMemsetAsync(sc.flag, 0, n, c->s);
     k_creep_grain<<<(rows + kCreepWarps - 1) / kCreepWarps, 32 * kCreepWarps, 0, c->s>>>(
