@@ -312,7 +312,8 @@ extern "C" hc_status hc_create(const hc_params* p, size_t max_bytes, hc_ctx** ou
   A(v.cin_x, (size_t)p->imax * p->jmax + 2) A(v.cin_y, (size_t)p->imax * p->jmax + 2)
   A(v.wet, N2) A(v.wet_sums, (N2 + 1023) / 1024 + 1)
   A(v.wet_bits, (size_t)p->imax * ((p->jmax + 31) / 32))
-  // partial sums: one per block of scan_area (32 x 8 cells) or of a grid_sum
+  // partial sums: one per block of a grid_sum, or of scan_area (32 x 64 cells; the
+  // capacity is that of blocks of 32 x 8)
   v.vpart_cap = (int)std::max<size_t>(
       (size_t)((p->jmax + 31) / 32) * (size_t)((p->imax + 7) / 8), 152 * 8);
   A(v.vpart, (size_t)v.vpart_cap)

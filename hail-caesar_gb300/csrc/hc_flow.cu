@@ -404,11 +404,6 @@ __global__ void k_flow_dt(const hc_view c, hc_dev* d) {
 // flow_route :3063-3247.  One thread per cell; cells outside the wet mask keep
 // their discharges (the reference does not visit them).
 // ---------------------------------------------------------------------------
-struct FaceOut {
-  double q, qs, vel;
-  int dir;  // 1: positive, -1: negative, 0: none
-};
-
 // The limiters' FP64 tests, for the faces whose float estimates cannot
 // decide them: out of line, so that their FP64 instructions (a hardware
 // division among them) issue only where they run.

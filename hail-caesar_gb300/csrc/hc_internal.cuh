@@ -49,8 +49,8 @@
 #define HC_ADJ_T1 (3 + HC_MAX_RF + 1)
 static_assert(HC_ADJ_REC == HC_ADJ_RECORD, "record size of the C ABI");
 
-// Device-side control block.  One per context, in device memory; the single
-// thread control kernel owns the scalar logic of the reference's driver.
+// Device-side control block.  One per context, in device memory; the control
+// kernel (one warp) owns the scalar logic of the reference's driver.
 struct hc_dev {
   hc_scalars s;           // scalar model state (mirrors LSDCatchmentModel)
   // per-iteration switches written by the control kernel
