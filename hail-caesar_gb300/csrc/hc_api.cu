@@ -1507,15 +1507,19 @@ static hc_status ensemble_group(hc_ctx** ctxs, const std::vector<int>& mine, int
                                 int32_t flags, int64_t* done) {
   std::vector<char> live(mine.size(), 0);
   int left = 0;
+  // a member's error ends that member's run; the others, whose graphs may be
+  // in flight, are served to their end
+  hc_status first = HC_OK;
+  auto failed = [&](hc_status st) {
+    if (st != HC_OK && first == HC_OK) first = st;
+    return st != HC_OK;
+  };
   for (size_t q = 0; q < mine.size(); q++) {
-    const int k = mine[q];
+    hc_ctx* c = ctxs[mine[q]];
     bool fin = false;
-    HC_TRY(run_begin(ctxs[k], n, flags, false, &fin));
-    if (!fin) {
-      HC_TRY(run_launch(ctxs[k]));
-      live[q] = 1;
-      left++;
-    }
+    if (failed(run_begin(c, n, flags, false, &fin)) || fin || failed(run_launch(c))) continue;
+    live[q] = 1;
+    left++;
   }
   while (left > 0) {
     bool progressed = false;
@@ -1525,21 +1529,23 @@ static hc_status ensemble_group(hc_ctx** ctxs, const std::vector<int>& mine, int
       hc_ctx* c = ctxs[k];
       const cudaError_t e = cudaEventQuery(c->chunk_done);
       if (e == cudaErrorNotReady) continue;
-      if (e != cudaSuccess) return hc_cuda(c, e, "ensemble");
       progressed = true;
       bool fin = false;
-      HC_TRY(run_after_chunk(c, flags, &fin));
+      if (failed(hc_cuda(c, e, "ensemble")) || failed(run_after_chunk(c, flags, &fin))) {
+        fin = true;
+      } else if (fin) {
+        failed(run_end(c, nullptr, done ? &done[k] : nullptr));
+      } else {
+        fin = failed(run_launch(c));
+      }
       if (fin) {
-        HC_TRY(run_end(c, nullptr, done ? &done[k] : nullptr));
         live[q] = 0;
         left--;
-      } else {
-        HC_TRY(run_launch(c));
       }
     }
     if (!progressed) std::this_thread::yield();
   }
-  return HC_OK;
+  return first;
 }
 
 // Members are shared out over host threads (member k to thread k mod T), so

@@ -326,7 +326,8 @@ hc_status hc_snapshot_end(hc_snapshot* snap);
  * differ in size and parameters.  The members are serviced by up to 32 host
  * threads (member k by thread k mod T), so one member's host-side step
  * holds up only the members of its thread; a member must not be used by
- * another thread during the call. */
+ * another thread during the call.  A member's error ends that member's run
+ * and is returned (the first, by thread) when the others are done. */
 hc_status hc_run_ensemble(hc_ctx** ctxs, int32_t m, int64_t n, int32_t flags, int64_t* done);
 
 /* ---- adjoint of the hydraulic iteration (no counterpart in the reference)
